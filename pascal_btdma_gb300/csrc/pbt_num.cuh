@@ -7,7 +7,7 @@
 //        error-free transformations TwoSum (Knuth, TAOCP vol. 2, 4.2.2),
 //        FastTwoSum (Dekker 1971) and the FMA form of TwoProduct (Ogita, Rump,
 //        Oishi, "Accurate sum and dot product", SIAM J. Sci. Comput. 26, 2005).
-//        Each multiply-accumulate costs 12 FP32 instructions, i.e. ~5x the
+//        Each multiply-accumulate costs 10 FP32 instructions, i.e. ~6x the
 //        FP64 pipe's rate.
 //   F32: plain float, the factorisation arithmetic of the iteratively refined
 //        solve (see k_residual64 in pbt_kernels.cuh).
@@ -125,51 +125,43 @@ struct FF {
     };
     static constexpr bool kConv = true;
 
-    // FP64 -> (h, l) by bit manipulation: h = x truncated to 24 significant
-    // bits, l = the next 23 bits, so |x - (h + l)| < 2^-46 |x|.  Only zero
-    // and magnitudes in the window [2^-96, 2^96) convert (kFFExpLo..kFFExpHi):
-    // there l is never below 2^-120, and a product of two such values stays
-    // inside FP32's range.  Anything else -- a nonzero |x| < 2^-96 (FP64
+    // FP64 -> (h, l): h = x truncated to 24 significant bits by bit
+    // manipulation, l = the 29 bits below them converted to float (rounded to
+    // 24 bits) and scaled by h's power of two, so |x - (h + l)| <= 2^-48 |x|.
+    // Only zero and magnitudes in the window [2^-96, 2^96) convert
+    // (kFFExpLo..kFFExpHi): there a product of two such values stays inside
+    // FP32's range.  Anything else -- a nonzero |x| < 2^-96 (FP64
     // subnormals read as zero), |x| >= 2^96, Inf, NaN -- becomes a NaN, which
     // every later operation carries into the solution, where the output check
     // (nonfinite) reports it: an input the arithmetic cannot carry gives a
     // reported failure, never a silently wrong number.
-    __device__ static __forceinline__ T split(double x) {
-        const unsigned hi = static_cast<unsigned>(__double2hiint(x));
-        const unsigned lo = static_cast<unsigned>(__double2loint(x));
-        const unsigned e = (hi >> 20) & 0x7ffu;
-        const unsigned sign = hi & 0x80000000u;
-        // h: rebias the exponent (1023 -> 127) and keep 23 mantissa bits.
-        const unsigned hb = __funnelshift_l(lo, (hi & 0x7fffffffu) - (896u << 20), 3) | sign;
-        // l: the 23 bits below h's mantissa as a float with an explicit leading
-        // one, minus that one (exact).
-        const unsigned eb = (e - 919u) << 23;
-        const float lf = __fsub_rn(__uint_as_float(eb | ((lo >> 6) & 0x7fffffu)), __uint_as_float(eb));
-        const unsigned lb = __float_as_uint(lf) | sign;
-        const bool in = (e - kFFExpLo) <= (kFFExpHi - kFFExpLo);
-        const unsigned out = (e != 0u) ? 0x7fc00000u : 0u;  // outside the window: NaN; zero: 0
-        return {__uint_as_float(in ? hb : out), __uint_as_float(in ? lb : 0u)};
-    }
+    __device__ static __forceinline__ T split(double x) { return split_range<kFFExpLo, kFFExpHi, 1u>(x); }
     // The same conversion without the window, for right-hand sides and the
     // library's own intermediates (the reduced rows of a segmented plan after
     // an FP64 sub-solve, a refinement residual): |x| < 2^-126 gives 0,
-    // 2^-126 <= |x| < 2^-103 keeps h only, |x| >= 2^128 and Inf/NaN give NaN.
+    // |x| >= 2^128 and Inf/NaN give NaN.
     // Entries that small are negligible next to the rest of a right-hand side
     // (the solve is linear in it), next to the reduced system's identity
     // diagonal blocks, or as the correction of a converged iterate; a whole
     // solution that small is caught by the output check, and an overflow is a
     // NaN in the solution.
-    __device__ static __forceinline__ T split_wide(double x) {
+    __device__ static __forceinline__ T split_wide(double x) { return split_range<897u, 1150u, 897u>(x); }
+    // Biased FP64 exponents Lo..Hi convert, those below Zero give 0, the rest
+    // NaN.  14 instructions (18 with the low word cut out by shifts, 23 bits
+    // of it, and an exponent window on the shifted field), 80 of these a row
+    // at m = 5.
+    template <unsigned Lo, unsigned Hi, unsigned Zero>
+    __device__ static __forceinline__ T split_range(double x) {
         const unsigned hi = static_cast<unsigned>(__double2hiint(x));
         const unsigned lo = static_cast<unsigned>(__double2loint(x));
-        const unsigned e = (hi >> 20) & 0x7ffu;
-        const unsigned sign = hi & 0x80000000u;
-        const unsigned hb = __funnelshift_l(lo, (hi & 0x7fffffffu) - (896u << 20), 3) | sign;
-        const unsigned eb = (e - 919u) << 23;
-        const float lf = __fsub_rn(__uint_as_float(eb | ((lo >> 6) & 0x7fffffu)), __uint_as_float(eb));
-        const unsigned lb = __float_as_uint(lf) | sign;
-        const unsigned h = (e > 1150u) ? 0x7fc00000u : (e > 896u ? hb : 0u);
-        return {__uint_as_float(h), __uint_as_float((e >= 920u && e <= 1150u) ? lb : 0u)};
+        const unsigned mag2 = hi << 1;  // exponent and the upper mantissa, without the sign
+        // Rebias the exponent (1023 -> 127) and keep 23 mantissa bits; the sign back on top.
+        const unsigned hb = (__funnelshift_l(lo, hi - (896u << 20), 3) & 0x7fffffffu) | (hi & 0x80000000u);
+        unsigned h = (mag2 - (Lo << 21) < ((Hi - Lo + 1u) << 21)) ? hb : 0x7fc00000u;
+        h = (mag2 < (Zero << 21)) ? 0u : h;
+        // Sign and power of two of h (0 for zero, Inf for NaN) times the bits below it.
+        const float l = __fmul_rn(__uint2float_rn(lo & 0x1fffffffu), __uint_as_float(h & 0xff800000u));
+        return {__uint_as_float(h), __fmul_rn(l, 0x1p-52f)};
     }
 
     // float -> double by bit manipulation: normal floats exactly, Inf and NaN
@@ -208,19 +200,32 @@ struct FF {
 
     __device__ static __forceinline__ Acc acc(T x) { return {x.h, x.l}; }
     __device__ static __forceinline__ Acc acc0() { return {0.f, 0.f}; }
-    // a += x*y: exact product of the high parts, the two cross terms folded
-    // into its error, the high sum by TwoSum, all errors into a.t.
+    // a += x*y in 10 instructions: s = a.s + p with p the rounded product of
+    // the high parts; TwoSum's split of s into a part v that came from p and
+    // the rest from a.s (both errors exact), with the error of p taken in the
+    // same FMA that forms p's error in the sum: fma(x.h, y.h, -v) = (p - v) +
+    // (x.h*y.h - p), rounded once.  The two cross terms join it, all errors
+    // go into a.t.  Separate TwoProduct and TwoSum take 12.  With the 14-
+    // instruction conversion and fin's FastTwoSum, which the issue-bound
+    // float-float kernels gain from alike (GB300, us a solve, before ->
+    // after): m = 5, 65536 x 256 5667 -> 5070, periodic 12112 -> 10591;
+    // m = 4, 256 x 32768 in 128 segments 4964 -> 4363; the error against
+    // 64-bit solutions is the same (9.9e-15 after 1.0e-14 on the first).
     __device__ static __forceinline__ void mac(Acc& a, T x, T y) {
-        const float p = __fmul_rn(x.h, y.h);
-        float e = __fmaf_rn(x.h, y.h, -p);
+        const float s = __fadd_rn(a.s, __fmul_rn(x.h, y.h));
+        const float v = __fsub_rn(s, a.s);
+        float e = __fmaf_rn(x.h, y.h, -v);
+        const float d = __fsub_rn(a.s, __fsub_rn(s, v));
         e = __fmaf_rn(x.h, y.l, e);
         e = __fmaf_rn(x.l, y.h, e);
-        const ff s = two_sum(a.s, p);
-        a.s = s.h;
-        a.t = __fadd_rn(a.t, __fadd_rn(s.l, e));
+        a.s = s;
+        a.t = __fadd_rn(a.t, __fadd_rn(e, d));
     }
     __device__ static __forceinline__ void msub(Acc& a, T x, T y) { mac(a, {-x.h, -x.l}, y); }
-    __device__ static __forceinline__ T fin(Acc a) { return two_sum(a.s, a.t); }
+    // FastTwoSum: a.s is a multiple of a.t's last place (its terms are larger
+    // than the rounding errors that a.t collects), except where cancellation
+    // has left fewer bits in a.t than the sum would lose.
+    __device__ static __forceinline__ T fin(Acc a) { return fast_two_sum(a.s, a.t); }
 
     __device__ static __forceinline__ T mul(T a, T b) {
         const float p = __fmul_rn(a.h, b.h);
