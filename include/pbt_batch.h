@@ -19,7 +19,7 @@
  * The solve runs, per block size present (largest total cost first), a
  * persistent launch over the local-stage items (the warp that completes a
  * tile's last segment also solves the tile's reduced system) and a
- * persistent launch over the update items, on the caller's stream; each
+ * launch over the update items, on the caller's stream; each
  * launch carries one block size's code.
  *
  * Tuning (pbt_batch_tuning): the number of segments of each tile is

@@ -20,6 +20,7 @@ struct pbt_batch {
     // items3; one persistent launch per block size present, in `order`.
     int off1[PBT_MAX_BLOCK + 1] = {}, cnt1[PBT_MAX_BLOCK + 1] = {};
     int off3[PBT_MAX_BLOCK + 1] = {}, cnt3[PBT_MAX_BLOCK + 1] = {};
+    int rows3[PBT_MAX_BLOCK + 1] = {};  // rows of the longest segment of items3
     std::vector<int> order;
     std::vector<long long> user_mat_off, user_vec_off;
     long long user_mat = 0, user_vec = 0, packed_mat = 0, packed_vec = 0, red_mat = 0, red_vec = 0;
@@ -33,7 +34,7 @@ struct pbt_batch {
     long long* d_user_vec_off = nullptr;
     long long* row_start = nullptr;
     long long pack_total = 0;
-    int* state = nullptr;  // error (always 0), pad, head1[m], head3[m] (kHeads each), seg_done[ntiles]
+    int* state = nullptr;  // error (always 0), pad, head1[m] (kHeads), seg_done[ntiles]
     unsigned long long* status = nullptr;
     double *aw = nullptr, *cw = nullptr, *ra = nullptr, *rc = nullptr, *rd = nullptr;
     cudaStream_t last_stream = nullptr;
@@ -45,7 +46,7 @@ namespace {
 constexpr unsigned kBatchMagic = 0x50425442u;
 constexpr int kHeads = PBT_MAX_BLOCK + 1;
 
-size_t state_ints(int ntiles) { return (size_t)2 + 2 * kHeads + (size_t)ntiles; }
+size_t state_ints(int ntiles) { return (size_t)2 + kHeads + (size_t)ntiles; }
 
 // One launch of the batch kernel for block size m (pbt_inst.cu instantiates
 // launch_batch per arithmetic and block size).
@@ -253,7 +254,9 @@ int pbt_batch_create(pbt_batch** out, int nsys, const int* m, const int* nrow, i
             items1.push_back(make_int2(i.t, i.s));
             if (i.s >= 0 && !seen[i.t]) {
                 seen[i.t] = 1;
-                for (int sg = 0; sg < tiles[i.t].nseg; ++sg) items3.push_back(make_int2(i.t, sg));
+                const auto& tl = tiles[i.t];
+                for (int sg = 0; sg < tl.nseg; ++sg) items3.push_back(make_int2(i.t, sg));
+                b->rows3[mm] = std::max(b->rows3[mm], (tl.rows + tl.nseg - 1) / tl.nseg);
             }
         }
         b->cnt1[mm] = (int)items1.size() - b->off1[mm];
@@ -375,7 +378,7 @@ int pbt_batch_solve(pbt_batch* b, const double* pa, const double* pb, const doub
     ba.tiles = b->tiles;
     ba.lane_rows = b->lane_rows;
     ba.status = b->status;
-    ba.seg_done = b->state + 2 + 2 * kHeads;
+    ba.seg_done = b->state + 2 + kHeads;
     b->last_grid = 0;
     for (int mm : b->order) {
         ba.items1 = b->items1 + b->off1[mm];
@@ -383,7 +386,7 @@ int pbt_batch_solve(pbt_batch* b, const double* pa, const double* pb, const doub
         ba.n1 = b->cnt1[mm];
         ba.n3 = b->cnt3[mm];
         ba.head1 = b->state + 2 + mm;
-        ba.head3 = b->state + 2 + kHeads + mm;
+        ba.rows3 = b->rows3[mm];
         int grid = 0;
         e = launch_m(b->precision, mm, ba, b->warps, s, &grid);
         if (e != cudaSuccess) return bcuda(e, "batch_solve: launch");

@@ -20,8 +20,8 @@
 //                   elimination of one segment of every lane), each writing
 //                   its two reduced rows; the warp that completes a tile's
 //                   last segment solves its 2P-row reduced system;
-//   k_batch_update  persistent over the stage-3 items (the interior update of
-//                   one segment of every lane).
+//   k_batch_update  the interior update, one warp per piece of a segment of
+//                   every lane.
 // The kernel boundaries order the stages, so no warp ever waits on another
 // (a tile's reduced system is solved by the warp that finishes it last, found
 // with an atomic counter).
@@ -210,35 +210,34 @@ __global__ void __launch_bounds__(batch_in_step<Num, M>() ? 32 * kBatchStepWarps
     report_status(ba.status, bad);
 }
 
+// One warp per piece of kUpdateRows rows of a (tile, segment) item: the rows
+// of a segment are independent (update_rows), so the items need no queue, and
+// few long segments fill the GPU too.  Against one warp a segment, the uneven
+// batch (32768 systems, N 16..4096, segments of 64 rows, float-float), us:
+// m = 5 812 -> 415, m = 4 513 -> 271, m = 3 473 -> 160, m = 2 206 -> 88.
 template <class Num, int M>
-__global__ void __launch_bounds__(128) k_batch_update(const BatchArgs ba) {
-    unsigned bad = 0;
-    while (true) {
-        const int item = warp_claim(ba.head3);
-        if (item >= ba.n3) break;
-        const int2 it = ba.items3[item];
-        const BatchTile tl = ba.tiles[it.x];
-        const int t = it.x, seg = it.y;
-        const int lane = threadIdx.x & 31;
-        const int n_lane = tl.rows;
-        if (lane < tl.lanes) {
-            const size_t plane = (size_t)32 * tl.rows, rs = 32;
-            const size_t mo = (size_t)tl.mat_off + lane, vo = (size_t)tl.vec_off + lane;
-            int f, l;
-            seg_rows(n_lane, tl.nseg, seg, f, l);
-            const size_t fo = (size_t)f * rs;
-            unsigned amax = 0;
-            update_body<Num, M>(ba.aw + mo + fo, ba.cw + mo + fo, ba.d + vo + fo, plane, rs, l - f + 1, true,
-                                ba.rd + tl.red_vec_off + lane, (size_t)32 * 2 * tl.nseg, rs, seg, amax);
-            bad |= range_bits<Num>(amax, false);
-        }
-    }
-    report_status(ba.status, bad);
+__global__ void __launch_bounds__(128, 4) k_batch_update(const BatchArgs ba, int pieces) {
+    const unsigned w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const unsigned item = w / (unsigned)pieces;
+    if (item >= (unsigned)ba.n3) return;
+    const int2 it = ba.items3[item];
+    const BatchTile tl = ba.tiles[it.x];
+    const int seg = it.y, lane = threadIdx.x & 31, q0 = (int)(w % (unsigned)pieces) * kUpdateRows;
+    int f, l;
+    seg_rows(tl.rows, tl.nseg, seg, f, l);
+    const int n = l - f + 1, q1 = min(n, q0 + kUpdateRows);
+    if (lane >= tl.lanes || q0 >= n) return;
+    const size_t plane = (size_t)32 * tl.rows, rs = 32;
+    const size_t mo = (size_t)tl.mat_off + lane + (size_t)f * rs, vo = (size_t)tl.vec_off + lane + (size_t)f * rs;
+    unsigned amax = 0;
+    update_rows<Num, M, true>(ba.aw + mo, ba.cw + mo, ba.d + vo, plane, rs, n, q0, q1, ba.rd + tl.red_vec_off + lane,
+                              (size_t)32 * 2 * tl.nseg, rs, seg, amax);
+    report_status(ba.status, range_bits<Num>(amax, false));
 }
 
-// The two launches of block size M on stream s, both persistent (as many
-// CTAs of `warps` warps as fit the device): the local stage with the reduced
-// solves, then the update.
+// The two launches of block size M on stream s: the local stage with the
+// reduced solves, persistent (as many CTAs of `warps` warps as fit the
+// device), then the update.
 template <class Num, int M>
 cudaError_t launch_batch(const BatchArgs& ba, int warps, cudaStream_t s, int* grid_out) {
     if constexpr (std::is_same<Num, F32>::value) {
@@ -258,10 +257,10 @@ cudaError_t launch_batch(const BatchArgs& ba, int warps, cudaStream_t s, int* gr
         if (grid_out) *grid_out = grid;
         if (ba.n1 > 0) k_batch_local<Num, M><<<grid, 32 * warps, smem, s>>>(ba);
         if (ba.n3 > 0) {
-            int per_sm3 = 0;
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm3, k_batch_update<Num, M>, 128, 0);
-            if (e != cudaSuccess) return e;
-            k_batch_update<Num, M><<<sms * (per_sm3 > 0 ? per_sm3 : 1), 128, 0, s>>>(ba);
+            const int pieces = (ba.rows3 + kUpdateRows - 1) / kUpdateRows;
+            const long long blocks = ((long long)ba.n3 * pieces + 3) / 4;
+            if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
+            k_batch_update<Num, M><<<(unsigned)blocks, 128, 0, s>>>(ba, pieces);
         }
         return cudaGetLastError();
     }

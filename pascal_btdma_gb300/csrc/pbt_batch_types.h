@@ -32,8 +32,8 @@ struct BatchArgs {
     const int2* items1;    // (tile, segment or -1 for a whole-line Thomas item)
     const int2* items3;    // (tile, segment)
     int n1, n3;
-    int* head1;            // queue heads, zeroed before every solve
-    int* head3;
+    int rows3;             // rows of the longest segment in items3
+    int* head1;            // queue head, zeroed before every solve
     int* seg_done;         // per tile: segments done (zeroed before every solve)
     unsigned long long* status;  // zero pivots, range flag
 };
