@@ -77,7 +77,7 @@ __device__ __forceinline__ void batch_modi(const BatchArgs& ba, const BatchTile&
 // 4-warp CTAs, 16.70 ms with 8.
 template <class Num, int M>
 __host__ __device__ constexpr bool batch_in_step() {
-    return rows_in_step<Num>() && modi_uses_lu<Num, M>();
+    return rows_in_step<Num>() && modi_uses_lu<Num, M>() && M <= 6;
 }
 constexpr int kBatchStepWarps = 8;
 
@@ -162,7 +162,7 @@ __device__ __forceinline__ void batch_stage1(const BatchArgs& ba, const BatchTil
 // the fused local stage of the other sizes keeps up to 255.
 template <class Num, int M>
 __host__ __device__ constexpr int batch_min_ctas() {
-    return batch_slots<Num, M>() > 0 ? 4 : 1;
+    return batch_slots<Num, M>() > 0 && M <= 6 ? 4 : 1;
 }
 
 template <class Num, int M>

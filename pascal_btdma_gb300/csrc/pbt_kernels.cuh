@@ -43,12 +43,14 @@
 
 namespace pbt {
 
-// Loop unrolling policy (PBT_UNROLL precedes every m x m loop): fully
-// unrolled by default, so the blocks live in registers.  A translation unit
-// instantiating only M = 7..10 defines PBT_UNROLL as "unroll 1" first: those
-// blocks do not fit in registers anyway, and full unrolling would only
-// multiply compile time (minutes per variant), so their loops stay rolled and
-// the blocks live in local memory.
+// Loop unrolling policy: the split row step (lu_factor, lu_solve and the
+// bodies built on them) is unrolled for every m, its one m x m block in
+// registers.  PBT_UNROLL precedes the loops of the fused forms, which hold
+// several blocks: fully unrolled by default; a translation unit instantiating
+// only M = 7..10 defines PBT_UNROLL as "unroll 1" first -- those blocks do not
+// fit in registers together, and unrolling would only multiply compile time --
+// so there the fused forms (the adjoint, the periodic reduced solve, FP32)
+// keep their blocks in local memory.
 #ifndef PBT_UNROLL
 #define PBT_UNROLL _Pragma("unroll")
 #endif
@@ -168,16 +170,45 @@ struct LU {
     unsigned swaps = 0;  // bit k: some thread of the warp swapped at step k
 };
 
+// step(k) for k = 0..M-1 or M-1..0, every step unrolled.  From m = 7 on the
+// steps exceed the compiler's limit on unrolled loops, and a loop left rolled
+// sends the block to local memory (m = 8: 512 bytes a thread): there k is a
+// compile-time constant of a recursion instead.
+template <int K>
+struct StepIndex {
+    __device__ constexpr operator int() const { return K; }
+};
+template <int K, int M, class F>
+__device__ __forceinline__ void steps_up(const F& step) {
+    if constexpr (M <= 6) {
+#pragma unroll
+        for (int k = 0; k < M; ++k) step(k);
+    } else if constexpr (K < M) {
+        step(StepIndex<K>{});
+        steps_up<K + 1, M>(step);
+    }
+}
+template <int K, int M, class F>
+__device__ __forceinline__ void steps_down(const F& step) {
+    if constexpr (M <= 6) {
+#pragma unroll
+        for (int k = M - 1; k >= 0; --k) step(k);
+    } else if constexpr (K >= 0) {
+        step(StepIndex<K>{});
+        steps_down<K - 1, M>(step);
+    }
+}
+
 template <class Num, int M>
 __device__ __forceinline__ void lu_factor(typename Num::Acc (&a)[M][M], LU<Num, M>& lu, unsigned& bad) {
     using T = typename Num::T;
     using Acc = typename Num::Acc;
-PBT_UNROLL
-    for (int k = 0; k < M; ++k) {
+    steps_up<0, M>([&](auto kc) {
+        const int k = kc;
         if (k + 1 < M) {
             int p = k;
             auto best = Num::akey(a[k][k]);
-PBT_UNROLL
+#pragma unroll
             for (int i = k + 1; i < M; ++i) {
                 const auto v = Num::akey(a[i][k]);
                 const bool gt = v > best;
@@ -186,10 +217,10 @@ PBT_UNROLL
             }
             if (__any_sync(__activemask(), p != k)) {
                 lu.swaps |= 1u << k;
-PBT_UNROLL
+#pragma unroll
                 for (int i = k + 1; i < M; ++i) {
                     const unsigned s = (p == i);
-PBT_UNROLL
+#pragma unroll
                     for (int c = k; c < M; ++c) {
                         const Acc t = a[k][c];
                         a[k][c] = Num::asel(s, a[i][c], t);
@@ -204,19 +235,19 @@ PBT_UNROLL
         const T r = Num::rcp(pv);
         lu.f[k][k] = r;
         T uk[M];
-PBT_UNROLL
+#pragma unroll
         for (int c = k + 1; c < M; ++c) {
             uk[c] = Num::fin(a[k][c]);
             lu.f[k][c] = uk[c];
         }
-PBT_UNROLL
+#pragma unroll
         for (int i = k + 1; i < M; ++i) {
             const T l = Num::mul(Num::fin(a[i][k]), r);
             lu.f[i][k] = l;
-PBT_UNROLL
+#pragma unroll
             for (int c = k + 1; c < M; ++c) Num::msub(a[i][c], l, uk[c]);
         }
-    }
+    });
 }
 
 // x = a^{-1} b for one column b (consumed) with the factors of lu_factor.
@@ -224,11 +255,11 @@ template <class Num, int M>
 __device__ __forceinline__ void lu_solve(const LU<Num, M>& lu, typename Num::Acc (&b)[M], typename Num::T (&x)[M]) {
     using T = typename Num::T;
     using Acc = typename Num::Acc;
-PBT_UNROLL
-    for (int k = 0; k < M; ++k) {
+    steps_up<0, M>([&](auto kc) {
+        const int k = kc;
         if (k + 1 < M && ((lu.swaps >> k) & 1u)) {
             const unsigned p = static_cast<unsigned>((lu.piv >> (4 * k)) & 15u);
-PBT_UNROLL
+#pragma unroll
             for (int i = k + 1; i < M; ++i) {
                 const unsigned s = (p == static_cast<unsigned>(i));
                 const Acc t = b[k];
@@ -238,16 +269,16 @@ PBT_UNROLL
         }
         const T bk = Num::fin(b[k]);
         b[k] = Num::acc(bk);
-PBT_UNROLL
+#pragma unroll
         for (int i = k + 1; i < M; ++i) Num::msub(b[i], lu.f[i][k], bk);
-    }
-PBT_UNROLL
-    for (int k = M - 1; k >= 0; --k) {
+    });
+    steps_down<M - 1, M>([&](auto kc) {
+        const int k = kc;
         const T xk = Num::mul(Num::fin(b[k]), lu.f[k][k]);
         x[k] = xk;
-PBT_UNROLL
+#pragma unroll
         for (int i = 0; i < k; ++i) Num::msub(b[i], lu.f[i][k], xk);
-    }
+    });
 }
 
 // ---------------------------------------------------------------------------
@@ -255,40 +286,40 @@ PBT_UNROLL
 // ---------------------------------------------------------------------------
 template <class Num, int M>
 __device__ __forceinline__ void in_blk(typename Num::T (&x)[M][M], const double* base, size_t plane) {
-PBT_UNROLL
+#pragma unroll
     for (int j = 0; j < M; ++j)
-PBT_UNROLL
+#pragma unroll
         for (int i = 0; i < M; ++i) x[i][j] = Num::in(base + (size_t)(i + M * j) * plane);
 }
 template <class Num, int M>
 __device__ __forceinline__ void in_blk_ro(typename Num::T (&x)[M][M], const double* base, size_t plane) {
-PBT_UNROLL
+#pragma unroll
     for (int j = 0; j < M; ++j)
-PBT_UNROLL
+#pragma unroll
         for (int i = 0; i < M; ++i) x[i][j] = Num::in_ro(base + (size_t)(i + M * j) * plane);
 }
 template <class Num, int M>
 __device__ __forceinline__ void ld_raw_blk(typename Num::T (&x)[M][M], const double* base, size_t plane) {
-PBT_UNROLL
+#pragma unroll
     for (int j = 0; j < M; ++j)
-PBT_UNROLL
+#pragma unroll
         for (int i = 0; i < M; ++i) x[i][j] = Num::lds(base + (size_t)(i + M * j) * plane);
 }
 template <class Num, int M>
 __device__ __forceinline__ void st_raw_blk(double* base, size_t plane, const typename Num::T (&x)[M][M]) {
-PBT_UNROLL
+#pragma unroll
     for (int j = 0; j < M; ++j)
-PBT_UNROLL
+#pragma unroll
         for (int i = 0; i < M; ++i) Num::sts(base + (size_t)(i + M * j) * plane, x[i][j]);
 }
 template <class Num, int M>
 __device__ __forceinline__ void ld_raw_vec(typename Num::T (&x)[M], const double* base, size_t plane) {
-PBT_UNROLL
+#pragma unroll
     for (int i = 0; i < M; ++i) x[i] = Num::lds(base + (size_t)i * plane);
 }
 template <class Num, int M>
 __device__ __forceinline__ void st_raw_vec(double* base, size_t plane, const typename Num::T (&x)[M]) {
-PBT_UNROLL
+#pragma unroll
     for (int i = 0; i < M; ++i) Num::sts(base + (size_t)i * plane, x[i]);
 }
 // Solution values: converted to FP64 on store, their largest magnitude
@@ -296,7 +327,7 @@ PBT_UNROLL
 // collected in `amax` for range_bits.
 template <class Num, int M>
 __device__ __forceinline__ void out_vec(double* base, size_t plane, const typename Num::T (&x)[M], unsigned& amax) {
-PBT_UNROLL
+#pragma unroll
     for (int i = 0; i < M; ++i) {
         Num::out(base + (size_t)i * plane, x[i]);
         amax = max(amax, Num::mag(x[i]));
@@ -309,9 +340,9 @@ __device__ __forceinline__ void st_fac_blk(double* base, size_t plane, const typ
     if (raw || !Num::kConv) {
         st_raw_blk<Num, M>(base, plane, x);
     } else {
-PBT_UNROLL
+#pragma unroll
         for (int j = 0; j < M; ++j)
-PBT_UNROLL
+#pragma unroll
             for (int i = 0; i < M; ++i) Num::out(base + (size_t)(i + M * j) * plane, x[i][j]);
     }
 }
@@ -335,18 +366,18 @@ __device__ __forceinline__ void ld_fac_blk(typename Num::T (&x)[M][M], const dou
     if (raw || !Num::kConv) {
         ld_raw_blk<Num, M>(x, base, plane);
     } else {
-PBT_UNROLL
+#pragma unroll
         for (int j = 0; j < M; ++j)
-PBT_UNROLL
+#pragma unroll
             for (int i = 0; i < M; ++i) x[i][j] = Num::in_rhs(base + (size_t)(i + M * j) * plane);
     }
 }
 
 template <class Num, int M>
 __device__ __forceinline__ void to_acc(typename Num::Acc (&d)[M][M], const typename Num::T (&s)[M][M]) {
-PBT_UNROLL
+#pragma unroll
     for (int i = 0; i < M; ++i)
-PBT_UNROLL
+#pragma unroll
         for (int j = 0; j < M; ++j) d[i][j] = Num::acc(s[i][j]);
 }
 
@@ -375,6 +406,12 @@ PBT_UNROLL
 #define PBT_ROW_FENCE 1
 #endif
 constexpr int kThomasThreads = PBT_THOMAS_THREADS;
+// Registers of the split-row-step kernels: from m = 7 on R alone takes
+// 2*m*m of them (98 .. 200), which a cap of 128 would send to local memory.
+template <int M>
+__host__ __device__ constexpr int lu_maxnreg() {
+    return M <= 6 ? PBT_THOMAS_MAXNREG : 255;
+}
 
 // Geometry of one solve as a body sees it: pointers already offset to the
 // thread's system (and segment), `plane` = element-plane stride, `rs` = row
@@ -465,8 +502,13 @@ PBT_UNROLL
 // thomas_body (fused gesv, every right-hand side in registers) for m <= 4,
 // where that fits the register budget and is the fastest form (GB300,
 // float-float m = 4, 131072 systems: 14.8 ms vs 17.0 ms split); thomas_body_lu
-// for m = 5, 6 (float-float m = 5, 65536 systems: 7.1 ms vs 8.6 ms fused);
-// thomas_body with local-memory blocks above.
+// from m = 5 on (float-float m = 5, 65536 systems: 7.1 ms vs 8.6 ms fused).
+// For m = 7..10 the fused form would keep its blocks in local memory; split,
+// with up to 255 registers a thread, against that (GB300, us): m = 8,
+// 16384 x 256 float-float 55522 -> 11397, FP64 56802 -> 16525; m = 10,
+// 16384 x 128 51831 -> 15183, 53324 -> 16434; in 4 segments (k_modi_lu) m = 8
+// 4096 x 1024 FP64 125000 -> 38000; periodic m = 8 16384 x 128 float-float
+// 108661 -> 9087.
 #ifndef PBT_THOMAS_LU_MIN
 #define PBT_THOMAS_LU_MIN 5
 #endif
@@ -485,9 +527,9 @@ PBT_UNROLL
 // A-column loops rolled; FP64 (smaller code, bound by its pipe) gains
 // nothing and keeps them unrolled.  A rolled A loop reads y_{q-1}[k] from
 // shared memory (cps slot M*M + k) instead of a register.
-template <class Num>
+template <class Num, int M>
 __host__ __device__ constexpr bool lu_rolled() {
-    return Num::kConv;
+    return Num::kConv || M > 6;
 }
 // Variants of the rolled float-float row, chosen by measurement (GB300,
 // pencil batch m = 5): the d column solved inside the C-column loop as its
@@ -519,7 +561,7 @@ __host__ __device__ constexpr bool lu_ldg() {
     return M == 6;
 }
 constexpr int kThomasLuMinBlock = PBT_THOMAS_LU_MIN;
-constexpr int kThomasLuMaxBlock = 6;
+constexpr int kThomasLuMaxBlock = PBT_MAX_BLOCK;
 // Whether the split-row-step kernels keep their CTA's warps in step row by
 // row (a barrier per row; InStep of thomas_body_lu / modi_body_lu).  Measured
 // on GB300 (m = 5): float-float issue is bound by instruction fetch, and
@@ -532,12 +574,10 @@ __host__ __device__ constexpr bool rows_in_step() {
     return std::is_same<Num, FF>::value;
 }
 // Which kernels run in step, by measurement (float-float, GB300): the split
-// row step (m = 5, 6) and the periodic solve up to m = 6 (m = 5 pencil batch
+// row step (m >= 5) and the periodic solve up to m = 6 (m = 5 pencil batch
 // of periodic lines 14.15 -> 12.09 ms); the fused forms up to m = 4, which
 // gain 1-2 % (m = 4: 65536 x 256 4.10 -> 4.01 ms, 256 lines of 32768 rows
-// in 128 segments 5.00 -> 4.94 ms).  From m = 7 on, where the fused forms keep
-// their blocks in local memory, the barrier costs 6-10 % (m = 8, 16384 x 256:
-// 57.5 -> 60.7 ms) and is left out, as in the adjoint (m = 4, 16384 lines
+// in 128 segments 5.00 -> 4.94 ms).  Not the adjoint (m = 4, 16384 lines
 // of 512 rows: 6.27 -> 6.85 ms with it).
 template <class Num, int M>
 __host__ __device__ constexpr bool fused_in_step() {
@@ -624,15 +664,15 @@ __device__ __forceinline__ void thomas_body_lu(const double* A, const double* B,
         {
             const size_t plane = opaque(plane0);
             const double* pd = D + o;
-PBT_UNROLL
+#pragma unroll
             for (int i = 0; i < M; ++i, pd += plane) xd[i] = Num::acc(Num::in_rhs(pd));
         }
         {
             const size_t plane = opaque(plane0);
             const double* pb = B + o;
-PBT_UNROLL
+#pragma unroll
             for (int j = 0; j < M; ++j)
-PBT_UNROLL
+#pragma unroll
                 for (int i = 0; i < M; ++i, pb += plane) r[i][j] = Num::acc(Num::in_ro(pb));
         }
         if (q > 0) {
@@ -642,30 +682,30 @@ PBT_UNROLL
             // used, so one column is always in flight.
             double an[M];
             if constexpr (lu_prefetch_a<Num, M>()) {
-PBT_UNROLL
+#pragma unroll
                 for (int i = 0; i < M; ++i, pa += plane) an[i] = __ldg(pa);
             }
-            constexpr int kKUnroll = lu_rolled<Num>() ? PBT_LU_K_UNROLL : M;
+            constexpr int kKUnroll = lu_rolled<Num, M>() ? PBT_LU_K_UNROLL : M;
 #pragma unroll(kKUnroll)
             for (int k = 0; k < M; ++k) {
                 T ck[M];
-PBT_UNROLL
+#pragma unroll
                 for (int j = 0; j < M; ++j) ck[j] = Num::lds(cps + (k * M + j) * cstride);
                 T yk;
-                if constexpr (lu_rolled<Num>())
+                if constexpr (lu_rolled<Num, M>())
                     yk = Num::lds(cps + (M * M + k) * cstride);
                 else
                     yk = y[k];
                 double ac[M];
                 if constexpr (lu_prefetch_a<Num, M>()) {
-PBT_UNROLL
+#pragma unroll
                     for (int i = 0; i < M; ++i) ac[i] = an[i];
                     if (k + 1 < M) {
-PBT_UNROLL
+#pragma unroll
                         for (int i = 0; i < M; ++i, pa += plane) an[i] = __ldg(pa);
                     }
                 }
-PBT_UNROLL
+#pragma unroll
                 for (int i = 0; i < M; ++i) {
                     T a;
                     if constexpr (lu_prefetch_a<Num, M>()) {
@@ -674,7 +714,7 @@ PBT_UNROLL
                         a = lu_ldg<M>() ? Num::in_ro(pa) : Num::in(pa);
                         pa += plane;
                     }
-PBT_UNROLL
+#pragma unroll
                     for (int j = 0; j < M; ++j) Num::msub(r[i][j], a, ck[j]);
                     Num::msub(xd[i], a, yk);
                 }
@@ -685,14 +725,14 @@ PBT_UNROLL
         lu_factor<Num, M>(r, lu, bad);
         // MergeY: y as column -1 of the rolled column loop (one copy of the
         // column solve's code for y and C).
-        if constexpr (MergeY && lu_rolled<Num>()) {
+        if constexpr (MergeY && lu_rolled<Num, M>()) {
             const size_t plane = opaque(plane0);
             const double* pc = C + o;
             double* pw = CW + o;
             auto ld_c = [&](const double* p) -> double { return (lu_ldg<M>() && raw) ? __ldg(p) : *p; };
             double nxt[M];
             if (lu_prefetch_c<Num, M>() && !last) {
-PBT_UNROLL
+#pragma unroll
                 for (int i = 0; i < M; ++i, pc += plane) nxt[i] = ld_c(pc);
             }
             const int jend = last ? 0 : M;
@@ -701,20 +741,20 @@ PBT_UNROLL
                 Acc cj[M];
                 T xj[M];
                 if (j < 0) {
-PBT_UNROLL
+#pragma unroll
                     for (int i = 0; i < M; ++i) cj[i] = xd[i];
                 } else if constexpr (lu_prefetch_c<Num, M>()) {
                     double cur[M];
-PBT_UNROLL
+#pragma unroll
                     for (int i = 0; i < M; ++i) cur[i] = nxt[i];
                     if (j + 1 < M) {
-PBT_UNROLL
+#pragma unroll
                         for (int i = 0; i < M; ++i, pc += plane) nxt[i] = ld_c(pc);
                     }
-PBT_UNROLL
+#pragma unroll
                     for (int i = 0; i < M; ++i) cj[i] = Num::acc(Num::in(&cur[i]));
                 } else {
-PBT_UNROLL
+#pragma unroll
                     for (int i = 0; i < M; ++i, pc += plane) {
                         const double v = ld_c(pc);
                         cj[i] = Num::acc(Num::in(&v));
@@ -722,13 +762,13 @@ PBT_UNROLL
                 }
                 lu_solve<Num, M>(lu, cj, xj);
                 if (j < 0) {
-PBT_UNROLL
+#pragma unroll
                     for (int i = 0; i < M; ++i) {
                         y[i] = xj[i];
                         Num::sts(cps + (M * M + i) * cstride, xj[i]);
                     }
                 } else {
-PBT_UNROLL
+#pragma unroll
                     for (int i = 0; i < M; ++i, pw += plane) {
                         if (raw || !Num::kConv)
                             Num::sts(pw, xj[i]);
@@ -747,8 +787,8 @@ PBT_UNROLL
             continue;
         }
         lu_solve<Num, M>(lu, xd, y);
-        if constexpr (lu_rolled<Num>()) {
-PBT_UNROLL
+        if constexpr (lu_rolled<Num, M>()) {
+#pragma unroll
             for (int k = 0; k < M; ++k) Num::sts(cps + (M * M + k) * cstride, y[k]);
         }
         {
@@ -770,33 +810,33 @@ PBT_UNROLL
         auto ld_c = [&](const double* p) -> double { return (lu_ldg<M>() && raw) ? __ldg(p) : *p; };
         double nxt[M];
         if constexpr (lu_prefetch_c<Num, M>()) {
-PBT_UNROLL
+#pragma unroll
             for (int i = 0; i < M; ++i, pc += plane) nxt[i] = ld_c(pc);
         }
-        constexpr int kColUnroll = lu_rolled<Num>() ? PBT_LU_COL_UNROLL : M;
+        constexpr int kColUnroll = lu_rolled<Num, M>() ? PBT_LU_COL_UNROLL : M;
 #pragma unroll(kColUnroll)
         for (int j = 0; j < M; ++j) {
             Acc cj[M];
             T xj[M];
             if constexpr (lu_prefetch_c<Num, M>()) {
                 double cur[M];
-PBT_UNROLL
+#pragma unroll
                 for (int i = 0; i < M; ++i) cur[i] = nxt[i];
                 if (j + 1 < M) {
-PBT_UNROLL
+#pragma unroll
                     for (int i = 0; i < M; ++i, pc += plane) nxt[i] = ld_c(pc);
                 }
-PBT_UNROLL
+#pragma unroll
                 for (int i = 0; i < M; ++i) cj[i] = Num::acc(Num::in(&cur[i]));
             } else {
-PBT_UNROLL
+#pragma unroll
                 for (int i = 0; i < M; ++i, pc += plane) {
                     const double v = ld_c(pc);
                     cj[i] = Num::acc(Num::in(&v));
                 }
             }
             lu_solve<Num, M>(lu, cj, xj);
-PBT_UNROLL
+#pragma unroll
             for (int i = 0; i < M; ++i, pw += plane) {
                 if (raw || !Num::kConv)
                     Num::sts(pw, xj[i]);
@@ -811,18 +851,32 @@ PBT_UNROLL
         if constexpr (InStep) cta_row_barrier();
         const size_t o = (size_t)q * rs;
         const size_t plane = opaque(plane0);
-        T c[M][M], t[M];
-        ld_fac_blk<Num, M>(c, CW + o, plane, raw);
-        ld_raw_vec<Num, M>(t, D + o, plane);
-PBT_UNROLL
-        for (int i = 0; i < M; ++i) {
-            Acc s = Num::acc(t[i]);
-PBT_UNROLL
-            for (int k = 0; k < M; ++k) Num::msub(s, c[i][k], y[k]);
-            t[i] = Num::fin(s);
+        if constexpr (M > 6) {
+            // Column by column of C': the block need not be held (each sum
+            // still takes its terms in ascending k).
+            Acc s[M];
+#pragma unroll
+            for (int i = 0; i < M; ++i) s[i] = Num::acc(Num::lds(D + o + (size_t)i * plane));
+#pragma unroll
+            for (int k = 0; k < M; ++k)
+#pragma unroll
+                for (int i = 0; i < M; ++i) Num::msub(s[i], ld_fac<Num>(CW + o + (size_t)(i + M * k) * plane, raw), y[k]);
+#pragma unroll
+            for (int i = 0; i < M; ++i) y[i] = Num::fin(s[i]);
+        } else {
+            T c[M][M], t[M];
+            ld_fac_blk<Num, M>(c, CW + o, plane, raw);
+            ld_raw_vec<Num, M>(t, D + o, plane);
+#pragma unroll
+            for (int i = 0; i < M; ++i) {
+                Acc s = Num::acc(t[i]);
+#pragma unroll
+                for (int k = 0; k < M; ++k) Num::msub(s, c[i][k], y[k]);
+                t[i] = Num::fin(s);
+            }
+#pragma unroll
+            for (int i = 0; i < M; ++i) y[i] = t[i];
         }
-PBT_UNROLL
-        for (int i = 0; i < M; ++i) y[i] = t[i];
         out_vec<Num, M>(D + o, plane, y, amax);
     }
     bad |= range_bits<Num>(amax, true);
@@ -842,7 +896,7 @@ static __device__ __noinline__ void thomas_idle_rows(int N) {
 }
 
 template <class Num, int M>
-__global__ void __maxnreg__(PBT_THOMAS_MAXNREG) k_thomas(const SolveArgs g) {
+__global__ void __maxnreg__(lu_maxnreg<M>()) k_thomas(const SolveArgs g) {
     constexpr bool kStep = thomas_in_step<Num, M>();
     const int sys = blockIdx.x * blockDim.x + threadIdx.x;
     if (sys >= g.nsys) {
@@ -868,7 +922,7 @@ __global__ void __maxnreg__(PBT_THOMAS_MAXNREG) k_thomas(const SolveArgs g) {
 // with the strides carried in SolveArgs) made the reference-layout solve ~5 %
 // slower.
 template <class Num, int M>
-__global__ void __maxnreg__(PBT_THOMAS_MAXNREG) k_thomas_lines(const SolveArgs g, const LineStrides ls) {
+__global__ void __maxnreg__(lu_maxnreg<M>()) k_thomas_lines(const SolveArgs g, const LineStrides ls) {
     constexpr bool kStep = thomas_in_step<Num, M>();
     const int sys = blockIdx.x * blockDim.x + threadIdx.x;
     if (sys >= g.nsys) {
@@ -916,14 +970,14 @@ template <int M, bool Ahead>
 __device__ __forceinline__ void ld_col_ahead(double (&cur)[M], double (&nxt)[M], const double*& pa, size_t plane,
                                              int k) {
     if constexpr (Ahead) {
-PBT_UNROLL
+#pragma unroll
         for (int i = 0; i < M; ++i) cur[i] = nxt[i];
         if (k + 1 < M) {
-PBT_UNROLL
+#pragma unroll
             for (int i = 0; i < M; ++i, pa += plane) nxt[i] = __ldg(pa);
         }
     } else {
-PBT_UNROLL
+#pragma unroll
         for (int i = 0; i < M; ++i, pa += plane) cur[i] = __ldg(pa);
     }
 }
@@ -944,7 +998,7 @@ __device__ __forceinline__ void thomas_cyclic_body(const double* A, const double
     // Column loops rolled for float-float (code size, as in thomas_body_lu)
     // and from m = 5 on in FP64 too: unrolled, the FP64 m = 5 body spills
     // ~0.6 KB a thread at the 128-register cap, rolled it spills nothing.
-    constexpr bool kRolled = lu_rolled<Num>() || M >= 5;
+    constexpr bool kRolled = lu_rolled<Num, M>() || M >= 5;
     // A's columns one ahead up to m = 5 (at m = 6 the extra registers spill).
     constexpr bool kPrefetchA = M <= 5;
     auto slot = [&](int s) -> double* { return cps + s * cstride; };
@@ -957,23 +1011,23 @@ __device__ __forceinline__ void thomas_cyclic_body(const double* A, const double
         if (q == 1) {
             const size_t plane = opaque(plane0);
             const double* pa = A + o;
-PBT_UNROLL
+#pragma unroll
             for (int j = 0; j < M; ++j)
-PBT_UNROLL
+#pragma unroll
                 for (int i = 0; i < M; ++i, pa += plane) Num::sts(slot(kE + i * M + j), Num::in(pa));
         } else {
             const size_t plane = opaque(plane0);
             const double* pa = A + o;
             Acc w[M][M];
-PBT_UNROLL
+#pragma unroll
             for (int i = 0; i < M; ++i)
-PBT_UNROLL
+#pragma unroll
                 for (int j = 0; j < M; ++j) w[i][j] = Num::acc0();
             // kPrefetchA: column k + 1 of A is loaded (raw) before column k
             // is used.
             double an[M];
             if constexpr (kPrefetchA) {
-PBT_UNROLL
+#pragma unroll
                 for (int i = 0; i < M; ++i, pa += plane) an[i] = __ldg(pa);
             }
 #pragma unroll(kRolled ? 1 : M)
@@ -981,34 +1035,34 @@ PBT_UNROLL
                 T ak[M], ek[M];
                 double ac[M];
                 ld_col_ahead<M, kPrefetchA>(ac, an, pa, plane, k);
-PBT_UNROLL
+#pragma unroll
                 for (int i = 0; i < M; ++i) ak[i] = Num::in(&ac[i]);
-PBT_UNROLL
+#pragma unroll
                 for (int j = 0; j < M; ++j) ek[j] = Num::lds(slot(kE + k * M + j));
-PBT_UNROLL
+#pragma unroll
                 for (int i = 0; i < M; ++i)
-PBT_UNROLL
+#pragma unroll
                     for (int j = 0; j < M; ++j) Num::mac(w[i][j], ak[i], ek[j]);
                 if (PBT_ROW_FENCE) mem_fence_compiler();
             }
-PBT_UNROLL
+#pragma unroll
             for (int i = 0; i < M; ++i)
-PBT_UNROLL
+#pragma unroll
                 for (int j = 0; j < M; ++j) Num::sts(slot(kE + i * M + j), Num::fin(w[i][j]));
         }
         Acc r[M][M], xd[M];
         {
             const size_t plane = opaque(plane0);
             const double* pd = D + o;
-PBT_UNROLL
+#pragma unroll
             for (int i = 0; i < M; ++i, pd += plane) xd[i] = Num::acc(Num::in_rhs(pd));
         }
         {
             const size_t plane = opaque(plane0);
             const double* pb = B + o;
-PBT_UNROLL
+#pragma unroll
             for (int j = 0; j < M; ++j)
-PBT_UNROLL
+#pragma unroll
                 for (int i = 0; i < M; ++i, pb += plane) r[i][j] = Num::acc(Num::in_ro(pb));
         }
         if (q > 1) {
@@ -1016,13 +1070,13 @@ PBT_UNROLL
             const double* pa = A + o;
             double an[M];
             if constexpr (kPrefetchA) {
-PBT_UNROLL
+#pragma unroll
                 for (int i = 0; i < M; ++i, pa += plane) an[i] = __ldg(pa);
             }
 #pragma unroll(kRolled ? 1 : M)
             for (int k = 0; k < M; ++k) {
                 T ck[M];
-PBT_UNROLL
+#pragma unroll
                 for (int j = 0; j < M; ++j) ck[j] = Num::lds(slot(k * M + j));
                 T yk;
                 if constexpr (kRolled)
@@ -1031,10 +1085,10 @@ PBT_UNROLL
                     yk = y[k];
                 double ac[M];
                 ld_col_ahead<M, kPrefetchA>(ac, an, pa, plane, k);
-PBT_UNROLL
+#pragma unroll
                 for (int i = 0; i < M; ++i) {
                     const T a = Num::in(&ac[i]);
-PBT_UNROLL
+#pragma unroll
                     for (int j = 0; j < M; ++j) Num::msub(r[i][j], a, ck[j]);
                     Num::msub(xd[i], a, yk);
                 }
@@ -1045,7 +1099,7 @@ PBT_UNROLL
         lu_factor<Num, M>(r, lu, bad);
         lu_solve<Num, M>(lu, xd, y);
         if constexpr (kRolled) {
-PBT_UNROLL
+#pragma unroll
             for (int k = 0; k < M; ++k) Num::sts(slot(kY + k), y[k]);
         }
         st_raw_vec<Num, M>(D + o, opaque(plane0), y);
@@ -1066,7 +1120,7 @@ PBT_UNROLL
                 Acc v[M];
                 T xj[M];
                 if (ecol) {
-PBT_UNROLL
+#pragma unroll
                     for (int i = 0; i < M; ++i) {
                         const T w = Num::lds(slot(kE + i * M + j));
                         if (last) {
@@ -1077,13 +1131,13 @@ PBT_UNROLL
                         }
                     }
                 } else {
-PBT_UNROLL
+#pragma unroll
                     for (int i = 0; i < M; ++i) v[i] = Num::acc(Num::in(pc + (size_t)i * plane));
                 }
                 lu_solve<Num, M>(lu, v, xj);
                 double* pw = (ecol ? EW : CW) + o + (size_t)(M * j) * plane;
                 const int s0 = ecol ? kE + j : j;
-PBT_UNROLL
+#pragma unroll
                 for (int i = 0; i < M; ++i) {
                     if (ecol || raw || !Num::kConv)
                         Num::sts(pw + (size_t)i * plane, xj[i]);
@@ -1098,9 +1152,9 @@ PBT_UNROLL
     }
     // Row 0 needs e'_{N-1} and y_{N-1} as the forward sweep left them: they
     // move to the C' and y slots, which the backward sweep does not use.
-PBT_UNROLL
+#pragma unroll
     for (int s = 0; s < M * M; ++s) Num::sts(slot(s), Num::lds(slot(kE + s)));
-PBT_UNROLL
+#pragma unroll
     for (int k = 0; k < M; ++k) Num::sts(slot(kY + k), y[k]);
     for (int q = N - 2; q >= 1; --q) {
         if constexpr (InStep) cta_row_barrier();
@@ -1109,14 +1163,14 @@ PBT_UNROLL
         T c[M][M], t[M];
         ld_fac_blk<Num, M>(c, CW + o, plane, raw);
         ld_raw_vec<Num, M>(t, D + o, plane);
-PBT_UNROLL
+#pragma unroll
         for (int i = 0; i < M; ++i) {
             Acc s = Num::acc(t[i]);
-PBT_UNROLL
+#pragma unroll
             for (int k = 0; k < M; ++k) Num::msub(s, c[i][k], y[k]);
             t[i] = Num::fin(s);
         }
-PBT_UNROLL
+#pragma unroll
         for (int i = 0; i < M; ++i) y[i] = t[i];
         st_raw_vec<Num, M>(D + o, plane, y);
         double* pe = EW + o;
@@ -1124,33 +1178,33 @@ PBT_UNROLL
         double en[M], ec[M];
         const double* pn = pe;
         if constexpr (kPrefetchA) {
-PBT_UNROLL
+#pragma unroll
             for (int i = 0; i < M; ++i, pn += plane) en[i] = *pn;
         }
 #pragma unroll(kRolled ? 1 : M)
         for (int j = 0; j < M; ++j) {
             T ej[M], nv[M];
-PBT_UNROLL
+#pragma unroll
             for (int k = 0; k < M; ++k) ej[k] = Num::lds(slot(kE + k * M + j));
             if constexpr (kPrefetchA) {
-PBT_UNROLL
+#pragma unroll
                 for (int i = 0; i < M; ++i) ec[i] = en[i];
                 if (j + 1 < M) {
-PBT_UNROLL
+#pragma unroll
                     for (int i = 0; i < M; ++i, pn += plane) en[i] = *pn;
                 }
             } else {
-PBT_UNROLL
+#pragma unroll
                 for (int i = 0; i < M; ++i, pn += plane) ec[i] = *pn;
             }
-PBT_UNROLL
+#pragma unroll
             for (int i = 0; i < M; ++i) {
                 Acc s = Num::acc(Num::from_raw(ec[i]));
-PBT_UNROLL
+#pragma unroll
                 for (int k = 0; k < M; ++k) Num::msub(s, c[i][k], ej[k]);
                 nv[i] = Num::fin(s);
             }
-PBT_UNROLL
+#pragma unroll
             for (int i = 0; i < M; ++i, pe += plane) {
                 Num::sts(pe, nv[i]);
                 Num::sts(slot(kE + i * M + j), nv[i]);
@@ -1169,15 +1223,15 @@ PBT_UNROLL
         {
             const size_t plane = opaque(plane0);
             const double* pd = D;
-PBT_UNROLL
+#pragma unroll
             for (int i = 0; i < M; ++i, pd += plane) t[i] = Num::acc(Num::in_rhs(pd));
             const double* pb = B;
-PBT_UNROLL
+#pragma unroll
             for (int j = 0; j < M; ++j)
-PBT_UNROLL
+#pragma unroll
                 for (int i = 0; i < M; ++i, pb += plane) r[i][j] = Num::acc(Num::in_ro(pb));
         }
-PBT_UNROLL
+#pragma unroll
         for (int h = 0; h < 2; ++h) {
             // h = 0: A_0 with e'_{N-1}, y_{N-1} (C' and y slots); h = 1: C_0
             // with e'_1 (e slots) and y_1 (registers).
@@ -1187,14 +1241,14 @@ PBT_UNROLL
 #pragma unroll(kRolled ? 1 : M)
             for (int k = 0; k < M; ++k) {
                 T ak[M], ek[M];
-PBT_UNROLL
+#pragma unroll
                 for (int i = 0; i < M; ++i, pa += plane) ak[i] = Num::in(pa);
-PBT_UNROLL
+#pragma unroll
                 for (int j = 0; j < M; ++j) ek[j] = Num::lds(slot(es + k * M + j));
                 const T yk = (h == 0) ? Num::lds(slot(kY + k)) : y[k];
-PBT_UNROLL
+#pragma unroll
                 for (int i = 0; i < M; ++i) {
-PBT_UNROLL
+#pragma unroll
                     for (int j = 0; j < M; ++j) Num::mac(r[i][j], ak[i], ek[j]);
                     Num::msub(t[i], ak[i], yk);
                 }
@@ -1213,10 +1267,10 @@ PBT_UNROLL
         T e[M][M], t[M];
         ld_raw_blk<Num, M>(e, EW + o, plane);
         ld_raw_vec<Num, M>(t, D + o, plane);
-PBT_UNROLL
+#pragma unroll
         for (int i = 0; i < M; ++i) {
             Acc s = Num::acc(t[i]);
-PBT_UNROLL
+#pragma unroll
             for (int k = 0; k < M; ++k) Num::mac(s, e[i][k], x0[k]);
             t[i] = Num::fin(s);
         }
@@ -1234,7 +1288,7 @@ static __device__ __noinline__ void cyclic_idle_rows(int N) {
 }
 
 template <class Num, int M>
-__global__ void __maxnreg__(PBT_THOMAS_MAXNREG) k_thomas_cyclic(const SolveArgs g) {
+__global__ void __maxnreg__(lu_maxnreg<M>()) k_thomas_cyclic(const SolveArgs g) {
     constexpr bool kStep = cyclic_in_step<Num, M>();
     const int sys = blockIdx.x * blockDim.x + threadIdx.x;
     if (sys >= g.nsys) {
@@ -1442,15 +1496,15 @@ PBT_UNROLL
 // accumulator block is live; R_q is factored once and d', the m columns of A'
 // and the m columns of C' are solved one column at a time (one rolled loop).
 // The backward sweep and the first row's step work column by column the same
-// way, with the carried row's A' and C' in the slots.  64-thread CTAs at 128
-// registers: 16 warps an SM where the shared memory allows.
+// way, with the carried row's A' and C' in the slots.  At m = 5, 6 64-thread
+// CTAs at 128 registers: 16 warps an SM where the shared memory allows.
 // Not for FP32 (the refined solve's corrections): its single-float values fit
 // the fused form's 255 registers with few spills, and the split form measured
 // slower there (pencil batch, P = 16, two FP32 solves per refined solve:
 // 23.4 ms against 18.2 ms).
 template <class Num, int M>
 __host__ __device__ constexpr bool modi_uses_lu() {
-    return M >= PBT_MODI_LU_MIN && M <= 6 && !std::is_same<Num, F32>::value;
+    return M >= PBT_MODI_LU_MIN && !std::is_same<Num, F32>::value;
 }
 
 template <class Num, int M, bool InStep = false>
@@ -1476,13 +1530,13 @@ __device__ __forceinline__ void modi_body_lu(const double* A, const double* B, c
             const size_t plane = opaque(plane0);
             const double* pa = A + o;
             Acc w[M][M];
-PBT_UNROLL
+#pragma unroll
             for (int i = 0; i < M; ++i)
-PBT_UNROLL
+#pragma unroll
                 for (int j = 0; j < M; ++j) w[i][j] = Num::acc0();
             double an[M];
             if constexpr (kPrefetchA) {
-PBT_UNROLL
+#pragma unroll
                 for (int i = 0; i < M; ++i, pa += plane) an[i] = __ldg(pa);
             }
 #pragma unroll 1
@@ -1490,31 +1544,31 @@ PBT_UNROLL
                 T ak[M], ek[M];
                 double ac[M];
                 ld_col_ahead<M, kPrefetchA>(ac, an, pa, plane, k);
-PBT_UNROLL
+#pragma unroll
                 for (int i = 0; i < M; ++i) ak[i] = Num::in(&ac[i]);
-PBT_UNROLL
+#pragma unroll
                 for (int j = 0; j < M; ++j) ek[j] = Num::lds(slot(kE + k * M + j));
-PBT_UNROLL
+#pragma unroll
                 for (int i = 0; i < M; ++i)
-PBT_UNROLL
+#pragma unroll
                     for (int j = 0; j < M; ++j) Num::mac(w[i][j], ak[i], ek[j]);
                 if (PBT_ROW_FENCE) mem_fence_compiler();
             }
-PBT_UNROLL
+#pragma unroll
             for (int i = 0; i < M; ++i)
-PBT_UNROLL
+#pragma unroll
                 for (int j = 0; j < M; ++j) Num::sts(slot(kE + i * M + j), Num::fin(w[i][j]));
         }
         Acc r[M][M], xd[M];
         {
             const size_t plane = opaque(plane0);
             const double* pd = D + o;
-PBT_UNROLL
+#pragma unroll
             for (int i = 0; i < M; ++i, pd += plane) xd[i] = Num::acc(Num::in_rhs(pd));
             const double* pb = B + o;
-PBT_UNROLL
+#pragma unroll
             for (int j = 0; j < M; ++j)
-PBT_UNROLL
+#pragma unroll
                 for (int i = 0; i < M; ++i, pb += plane) r[i][j] = Num::acc(Num::in_ro(pb));
         }
         if (!first2) {
@@ -1522,21 +1576,21 @@ PBT_UNROLL
             const double* pa = A + o;
             double an[M];
             if constexpr (kPrefetchA) {
-PBT_UNROLL
+#pragma unroll
                 for (int i = 0; i < M; ++i, pa += plane) an[i] = __ldg(pa);
             }
 #pragma unroll 1
             for (int k = 0; k < M; ++k) {
                 T ck[M];
-PBT_UNROLL
+#pragma unroll
                 for (int j = 0; j < M; ++j) ck[j] = Num::lds(slot(k * M + j));
                 const T yk = Num::lds(slot(kY + k));
                 double ac[M];
                 ld_col_ahead<M, kPrefetchA>(ac, an, pa, plane, k);
-PBT_UNROLL
+#pragma unroll
                 for (int i = 0; i < M; ++i) {
                     const T a = Num::in(&ac[i]);
-PBT_UNROLL
+#pragma unroll
                     for (int j = 0; j < M; ++j) Num::msub(r[i][j], a, ck[j]);
                     Num::msub(xd[i], a, yk);
                 }
@@ -1546,7 +1600,7 @@ PBT_UNROLL
         LU<Num, M> lu;
         lu_factor<Num, M>(r, lu, bad);
         lu_solve<Num, M>(lu, xd, y);
-PBT_UNROLL
+#pragma unroll
         for (int k = 0; k < M; ++k) Num::sts(slot(kY + k), y[k]);
         st_raw_vec<Num, M>(D + o, opaque(plane0), y);
         // jj < m: column jj of A' (right-hand side A on rows 0, 1, else -W);
@@ -1561,17 +1615,17 @@ PBT_UNROLL
                 Acc v[M];
                 T xj[M];
                 if (acol && !first2) {
-PBT_UNROLL
+#pragma unroll
                     for (int i = 0; i < M; ++i) v[i] = Num::acc(Num::neg(Num::lds(slot(kE + i * M + j))));
                 } else {
                     const double* ps = (acol ? A : C) + co;
-PBT_UNROLL
+#pragma unroll
                     for (int i = 0; i < M; ++i) v[i] = Num::acc(Num::in(ps + (size_t)i * plane));
                 }
                 lu_solve<Num, M>(lu, v, xj);
                 double* pw = (acol ? AW : CW) + co;
                 const int s0 = acol ? kE + j : j;
-PBT_UNROLL
+#pragma unroll
                 for (int i = 0; i < M; ++i) {
                     st_fac<Num>(pw + (size_t)i * plane, xj[i], raw);
                     Num::sts(slot(s0 + i * M), xj[i]);
@@ -1583,9 +1637,9 @@ PBT_UNROLL
     // Reduced row 2*seg+1 = the segment's last row (A'_n, C'_n, d'_n).
     {
         const size_t ro = rrs * (size_t)(2 * seg + 1);
-PBT_UNROLL
+#pragma unroll
         for (int j = 0; j < M; ++j)
-PBT_UNROLL
+#pragma unroll
             for (int i = 0; i < M; ++i) {
                 Num::sts(RA + ro + (size_t)(i + M * j) * rplane, Num::lds(slot(kE + i * M + j)));
                 Num::sts(RC + ro + (size_t)(i + M * j) * rplane, Num::lds(slot(i * M + j)));
@@ -1598,9 +1652,9 @@ PBT_UNROLL
         const int q1 = (n >= 4) ? n - 2 : 1;
         const size_t o1 = (size_t)q1 * rs;
         const size_t plane = opaque(plane0);
-PBT_UNROLL
+#pragma unroll
         for (int j = 0; j < M; ++j)
-PBT_UNROLL
+#pragma unroll
             for (int i = 0; i < M; ++i) {
                 const size_t e = (size_t)(i + M * j) * plane;
                 Num::sts(slot(kE + i * M + j), ld_fac<Num>(AW + o1 + e, raw));
@@ -1615,14 +1669,14 @@ PBT_UNROLL
         T c[M][M], t[M];
         ld_fac_blk<Num, M>(c, CW + o, plane, raw);
         ld_raw_vec<Num, M>(t, D + o, plane);
-PBT_UNROLL
+#pragma unroll
         for (int i = 0; i < M; ++i) {
             Acc s = Num::acc(t[i]);
-PBT_UNROLL
+#pragma unroll
             for (int k = 0; k < M; ++k) Num::msub(s, c[i][k], y[k]);
             t[i] = Num::fin(s);
         }
-PBT_UNROLL
+#pragma unroll
         for (int i = 0; i < M; ++i) y[i] = t[i];
         st_raw_vec<Num, M>(D + o, plane, y);
 #pragma unroll 1
@@ -1632,16 +1686,16 @@ PBT_UNROLL
             const int s0 = acol ? kE + j : j;
             double* pw = (acol ? AW : CW) + o + (size_t)(M * j) * plane;
             T cj[M], nv[M];
-PBT_UNROLL
+#pragma unroll
             for (int k = 0; k < M; ++k) cj[k] = Num::lds(slot(s0 + k * M));
-PBT_UNROLL
+#pragma unroll
             for (int i = 0; i < M; ++i) {
                 Acc s = acol ? Num::acc(ld_fac<Num>(pw + (size_t)i * plane, raw)) : Num::acc0();
-PBT_UNROLL
+#pragma unroll
                 for (int k = 0; k < M; ++k) Num::msub(s, c[i][k], cj[k]);
                 nv[i] = Num::fin(s);
             }
-PBT_UNROLL
+#pragma unroll
             for (int i = 0; i < M; ++i) {
                 st_fac<Num>(pw + (size_t)i * plane, nv[i], raw);
                 Num::sts(slot(s0 + i * M), nv[i]);
@@ -1656,50 +1710,50 @@ PBT_UNROLL
     // its slots first.
     {
         const size_t plane = opaque(plane0);
-PBT_UNROLL
+#pragma unroll
         for (int k = 0; k < M; ++k) Num::sts(slot(kY + k), y[k]);
         {
             Acc w[M][M];
-PBT_UNROLL
+#pragma unroll
             for (int i = 0; i < M; ++i)
-PBT_UNROLL
+#pragma unroll
                 for (int j = 0; j < M; ++j) w[i][j] = Num::acc0();
 #pragma unroll 1
             for (int k = 0; k < M; ++k) {
                 T ck[M], ek[M];
-PBT_UNROLL
+#pragma unroll
                 for (int i = 0; i < M; ++i) ck[i] = ld_fac<Num>(CW + (size_t)(i + M * k) * plane, raw);
-PBT_UNROLL
+#pragma unroll
                 for (int j = 0; j < M; ++j) ek[j] = Num::lds(slot(k * M + j));
-PBT_UNROLL
+#pragma unroll
                 for (int i = 0; i < M; ++i)
-PBT_UNROLL
+#pragma unroll
                     for (int j = 0; j < M; ++j) Num::mac(w[i][j], ck[i], ek[j]);
                 if (PBT_ROW_FENCE) mem_fence_compiler();
             }
-PBT_UNROLL
+#pragma unroll
             for (int i = 0; i < M; ++i)
-PBT_UNROLL
+#pragma unroll
                 for (int j = 0; j < M; ++j) Num::sts(slot(i * M + j), Num::fin(w[i][j]));
         }
         Acc r[M][M], xd[M];
-PBT_UNROLL
+#pragma unroll
         for (int i = 0; i < M; ++i) {
             xd[i] = Num::acc(Num::lds(D + (size_t)i * plane));
-PBT_UNROLL
+#pragma unroll
             for (int j = 0; j < M; ++j) r[i][j] = Num::acc(i == j ? Num::one() : Num::zero());
         }
 #pragma unroll 1
         for (int k = 0; k < M; ++k) {
             T ck[M], ek[M];
-PBT_UNROLL
+#pragma unroll
             for (int i = 0; i < M; ++i) ck[i] = ld_fac<Num>(CW + (size_t)(i + M * k) * plane, raw);
-PBT_UNROLL
+#pragma unroll
             for (int j = 0; j < M; ++j) ek[j] = Num::lds(slot(kE + k * M + j));
             const T yk = Num::lds(slot(kY + k));
-PBT_UNROLL
+#pragma unroll
             for (int i = 0; i < M; ++i) {
-PBT_UNROLL
+#pragma unroll
                 for (int j = 0; j < M; ++j) Num::msub(r[i][j], ck[i], ek[j]);
                 Num::msub(xd[i], ck[i], yk);
             }
@@ -1718,13 +1772,13 @@ PBT_UNROLL
             double* pw = (acol ? AW : CW) + (size_t)(M * j) * plane;
             Acc v[M];
             T xj[M];
-PBT_UNROLL
+#pragma unroll
             for (int i = 0; i < M; ++i)
                 v[i] = acol ? Num::acc(ld_fac<Num>(pw + (size_t)i * plane, raw))
                             : Num::acc(Num::neg(Num::lds(slot(j + i * M))));
             lu_solve<Num, M>(lu, v, xj);
             double* pr = (acol ? RA : RC) + ro + (size_t)(M * j) * rplane;
-PBT_UNROLL
+#pragma unroll
             for (int i = 0; i < M; ++i) {
                 st_fac<Num>(pw + (size_t)i * plane, xj[i], raw);
                 Num::sts(pr + (size_t)i * rplane, xj[i]);
@@ -1742,7 +1796,7 @@ static __device__ __noinline__ void modi_idle_rows(int n) {
 }
 
 template <class Num, int M>
-__global__ void __maxnreg__(PBT_THOMAS_MAXNREG) k_modi_lu(const SolveArgs g) {
+__global__ void __maxnreg__(lu_maxnreg<M>()) k_modi_lu(const SolveArgs g) {
     constexpr bool kStep = rows_in_step<Num>();
     const int sys = blockIdx.x * blockDim.x + threadIdx.x;
     const int seg = blockIdx.y;
@@ -1886,11 +1940,11 @@ __device__ __forceinline__ void reduced_body_lu(const double* RA, double* RC, do
     {
         // Row 0: B = I, so [C'|y] = [C|d] exactly.
         const size_t plane = opaque(plane0);
-PBT_UNROLL
+#pragma unroll
         for (int j = 0; j < M; ++j)
-PBT_UNROLL
+#pragma unroll
             for (int i = 0; i < M; ++i) Num::sts(slot(i * M + j), Num::lds(RC + (size_t)(i + M * j) * plane));
-PBT_UNROLL
+#pragma unroll
         for (int i = 0; i < M; ++i) {
             y[i] = Num::lds(RD + (size_t)i * plane);
             Num::sts(slot(kY + i), y[i]);
@@ -1902,24 +1956,24 @@ PBT_UNROLL
         Acc r[M][M], xd[M];
         {
             const size_t plane = opaque(plane0);
-PBT_UNROLL
+#pragma unroll
             for (int i = 0; i < M; ++i) {
                 xd[i] = Num::acc(Num::lds(RD + o + (size_t)i * plane));
-PBT_UNROLL
+#pragma unroll
                 for (int j = 0; j < M; ++j) r[i][j] = Num::acc(i == j ? Num::one() : Num::zero());
             }
             const double* pa = RA + o;
 #pragma unroll 1
             for (int k = 0; k < M; ++k) {
                 T ck[M], ak[M];
-PBT_UNROLL
+#pragma unroll
                 for (int j = 0; j < M; ++j) ck[j] = Num::lds(slot(k * M + j));
                 const T yk = Num::lds(slot(kY + k));
-PBT_UNROLL
+#pragma unroll
                 for (int i = 0; i < M; ++i, pa += plane) ak[i] = Num::lds(pa);
-PBT_UNROLL
+#pragma unroll
                 for (int i = 0; i < M; ++i) {
-PBT_UNROLL
+#pragma unroll
                     for (int j = 0; j < M; ++j) Num::msub(r[i][j], ak[i], ck[j]);
                     Num::msub(xd[i], ak[i], yk);
                 }
@@ -1932,17 +1986,17 @@ PBT_UNROLL
         const size_t plane = opaque(plane0);
         st_raw_vec<Num, M>(RD + o, plane, y);
         if (last) break;
-PBT_UNROLL
+#pragma unroll
         for (int k = 0; k < M; ++k) Num::sts(slot(kY + k), y[k]);
 #pragma unroll 1
         for (int j = 0; j < M; ++j) {
             double* pc = RC + o + (size_t)(M * j) * plane;
             Acc cj[M];
             T xj[M];
-PBT_UNROLL
+#pragma unroll
             for (int i = 0; i < M; ++i) cj[i] = Num::acc(Num::lds(pc + (size_t)i * plane));
             lu_solve<Num, M>(lu, cj, xj);
-PBT_UNROLL
+#pragma unroll
             for (int i = 0; i < M; ++i) {
                 Num::sts(pc + (size_t)i * plane, xj[i]);
                 Num::sts(slot(i * M + j), xj[i]);
@@ -1952,7 +2006,7 @@ PBT_UNROLL
     }
     // Backward, as reduced_body, with its range check of the line.
     unsigned amax = 0;
-PBT_UNROLL
+#pragma unroll
     for (int i = 0; i < M; ++i) amax = max(amax, Num::mag(y[i]));
     for (int q = R - 2; q >= 0; --q) {
         const size_t o = (size_t)q * rs;
@@ -1960,28 +2014,39 @@ PBT_UNROLL
         T c[M][M], t[M];
         ld_raw_blk<Num, M>(c, RC + o, plane);
         ld_raw_vec<Num, M>(t, RD + o, plane);
-PBT_UNROLL
+#pragma unroll
         for (int i = 0; i < M; ++i) {
             Acc s = Num::acc(t[i]);
-PBT_UNROLL
+#pragma unroll
             for (int k = 0; k < M; ++k) Num::msub(s, c[i][k], y[k]);
             t[i] = Num::fin(s);
             amax = max(amax, Num::mag(t[i]));
         }
-PBT_UNROLL
+#pragma unroll
         for (int i = 0; i < M; ++i) y[i] = t[i];
         st_raw_vec<Num, M>(RD + o, plane, y);
     }
     bad |= range_bits<Num>(amax, true);
 }
 
+// From m = 7 on the fused form keeps its blocks in local memory.
+template <int M>
+__host__ __device__ constexpr bool reduced_uses_lu() {
+    return M > 6;
+}
 template <class Num, int M>
 __global__ void __launch_bounds__(128) k_reduced(const SolveArgs g) {
     const int sys = blockIdx.x * blockDim.x + threadIdx.x;
     if (sys >= g.nsys) return;
     unsigned bad = 0;
     const size_t rs = (size_t)g.nsys;
-    reduced_body<Num, M>(g.ra + sys, g.rc + sys, g.rd + sys, rs * 2 * g.nseg, rs, 2 * g.nseg, bad);
+    if constexpr (reduced_uses_lu<M>()) {
+        extern __shared__ double thomas_cps[];
+        reduced_body_lu<Num, M>(g.ra + sys, g.rc + sys, g.rd + sys, thomas_cps + threadIdx.x, blockDim.x,
+                                rs * 2 * g.nseg, rs, 2 * g.nseg, bad);
+    } else {
+        reduced_body<Num, M>(g.ra + sys, g.rc + sys, g.rd + sys, rs * 2 * g.nseg, rs, 2 * g.nseg, bad);
+    }
     report_status(g.status, bad);
 }
 
@@ -2759,7 +2824,9 @@ cudaError_t launch_modi(const SolveArgs& g) {
 }
 template <class Num, int M>
 cudaError_t launch_reduced(const SolveArgs& g) {
-    k_reduced<Num, M><<<grid_x(g.nsys, g.tpb), g.tpb, 0, g.stream>>>(g);
+    const int tpb = reduced_uses_lu<M>() && g.tpb > 32 ? 32 : g.tpb;
+    const size_t smem = reduced_uses_lu<M>() ? (size_t)tpb * (M * M + M) * sizeof(double) : 0;  // <= 28.2 KB
+    k_reduced<Num, M><<<grid_x(g.nsys, tpb), tpb, smem, g.stream>>>(g);
     return cudaGetLastError();
 }
 template <class Num, int M>

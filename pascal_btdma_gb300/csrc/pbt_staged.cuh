@@ -103,7 +103,7 @@ __device__ __forceinline__ void fence_proxy_async_global() { asm volatile("fence
 // of a rolled loop costs more than the smaller code saves.
 template <class Num, int M>
 __host__ __device__ constexpr bool staged_rolled() {
-    return lu_rolled<Num>() && sizeof(typename Num::T) == 8 && M == 4;
+    return lu_rolled<Num, M>() && sizeof(typename Num::T) == 8 && M == 4;
 }
 // Shared memory of one CTA: the ring (R items of M*32 doubles), C'_{q-1}
 // (M*M*32 raw values) and, with rolled loops, y_{q-1} (M*32).  Sized so that
