@@ -318,7 +318,55 @@ bool thomas_stages(const pbt_plan* p, int arith, int m, const pbt::SolveArgs& g,
                           : encode_columns(&maps->w, g.cw, g.nsys, g.nrow, mm, m));
 }
 
+cudaError_t run_thomas_cols(int arith, int m, const pbt::SolveArgs& g, const pbt::LineStrides& ls) {
+    if (arith == kFF) {
+        PBT_DISPATCH_PLAIN_M2(pbt::FF, launch_thomas_cols, g, ls)
+    }
+    PBT_DISPATCH_PLAIN_M2(pbt::F64, launch_thomas_cols, g, ls)
+}
+cudaError_t run_modi_cols(int arith, int m, const pbt::SolveArgs& g) {
+    if (arith == kFF) {
+        PBT_DISPATCH_PLAIN_M2(pbt::FF, launch_modi_cols, g)
+    }
+    PBT_DISPATCH_PLAIN_M2(pbt::F64, launch_modi_cols, g)
+}
+cudaError_t run_reduced_cols(int arith, int m, const pbt::SolveArgs& g) {
+    if (arith == kFF) {
+        PBT_DISPATCH_PLAIN_M2(pbt::FF, launch_reduced_cols, g)
+    }
+    PBT_DISPATCH_PLAIN_M2(pbt::F64, launch_reduced_cols, g)
+}
+
+// Whether `items` systems (or, with `local`, segments of the local stage) are
+// so few that one lane per block column (pbt_cols.cuh) beats one thread per
+// item, whose threads per SM they would be; the bits are the same.  From
+// sweeps on GB300 (152 SMs; us, one thread -> one lane a column, on both sides
+// of the line):
+//   FP64, line at 70 threads an SM (10640 systems x 64 rows), 90 for m <= 3 and
+//     the local stage: m = 3 12288 425 -> 371, 16384 441 -> 485; m = 5 1024
+//     1236 -> 361, 10240 1249 -> 1109, 12288 1249 -> 1443; m = 8 10240 4090 ->
+//     3829, 12288 4108 -> 5626; m = 10 4096 7986 -> 3999, 8192 7985 -> 8464
+//     (line at 45); local stage 3, 1024 x 128 in 4 342 -> 176,
+//     4, 2048 x 512 in 8 1567 -> 1761;
+//   float-float, line at 180 (27360), 384 for m <= 3: m = 3 16384 373 -> 170,
+//     65536 534 -> 514; m = 5 4096 723 -> 230, 24000 850 -> 781, 32768 913 ->
+//     1049; m = 8 24000 3295 -> 3002, 32768 3403 -> 4157; local stage 5,
+//     2048 x 256 in 8 1230 -> 695, 6, 2048 x 512 in 16 2829 -> 3243.
+// FP64 leaves first: its pipe is full with fewer warps, and the extra
+// multiply-adds in idle slots count from then on.
+bool cols_pay(int arith, int m, long long items, bool local, int sms) {
+    if (arith == kF32 || m > pbt::kColsMaxBlock) return false;
+    const int line = arith == kFF ? (!local && m <= 3 ? 384 : 180) : (local || m <= 3 ? 90 : m <= 9 ? 70 : 45);
+    return items < (long long)line * (sms > 0 ? sms : 1);
+}
+bool thomas_cols(const pbt_plan* p, int arith, int m) {
+    return !(p->desc.flags & (PBT_FLAG_DIRECT_LOADS | PBT_FLAG_STAGED_LOADS)) &&
+           cols_pay(arith, m, p->desc.nsys, false, p->sms);
+}
+
 cudaError_t thomas_launch(const pbt_plan* p, int arith, int m, const pbt::SolveArgs& g) {
+    if (thomas_cols(p, arith, m))
+        return run_thomas_cols(arith, m, g, {g.nsys, 1, 0, g.nsys, (long long)g.nsys * g.nrow});
     pbt::ThomasMaps maps;
     return thomas_stages(p, arith, m, g, &maps) ? run_thomas_staged(arith, m, g, maps) : run_thomas(arith, m, g);
 }
@@ -354,6 +402,16 @@ PBT_DISPATCH(run_modi, launch_modi)
 PBT_DISPATCH(run_reduced, launch_reduced)
 PBT_DISPATCH(run_reduced_cyclic, launch_reduced_cyclic)
 PBT_DISPATCH(run_update, launch_update)
+
+// Stages 1 and 2 of the two-stage method, each with one thread or one lane per
+// block column as its items ask.
+cudaError_t local_launch(const pbt_plan* p, int arith, int m, const pbt::SolveArgs& g) {
+    return cols_pay(arith, m, (long long)g.nsys * g.nseg, true, p->sms) ? run_modi_cols(arith, m, g)
+                                                                         : run_modi(arith, m, g);
+}
+cudaError_t reduced_launch(const pbt_plan* p, int arith, int m, const pbt::SolveArgs& g) {
+    return cols_pay(arith, m, g.nsys, false, p->sms) ? run_reduced_cols(arith, m, g) : run_reduced(arith, m, g);
+}
 
 // Whether a batch fills the GPU with one thread per system: at least 4 warps
 // per SM.  Measured on GB300: the m = 5 pencil batch (65536 systems, 13.5
@@ -532,8 +590,8 @@ int solve_refined(pbt_plan* p, double* a, double* b, double* c, double* d, cudaS
     auto fp32_solve = [&](double* rhs) -> cudaError_t {
         if (p->thomas) return thomas_launch(p, kF32, m, make_args(p, a, b, c, rhs, s, ds.nsys));
         pbt::SolveArgs g = make_args(p, a, b, c, rhs, s, ds.nsys * ds.nseg);
-        cudaError_t e = run_modi(kF32, m, g);
-        if (e == cudaSuccess) e = run_reduced(kF32, m, make_args(p, a, b, c, rhs, s, ds.nsys));
+        cudaError_t e = local_launch(p, kF32, m, g);
+        if (e == cudaSuccess) e = reduced_launch(p, kF32, m, make_args(p, a, b, c, rhs, s, ds.nsys));
         if (e == cudaSuccess) e = run_update(kF32, m, g);
         return e;
     };
@@ -683,7 +741,7 @@ int solve_core(pbt_plan* p, double* a, double* b, double* c, double* d, int m, i
             if ((e = mark(i)) != cudaSuccess) return cuda_fail(e, "cudaEventRecord");
     } else {
         pbt::SolveArgs g = make_args(p, a, b, c, d, s, nsys * ds.nseg);
-        e = run_modi(arith_of(ds.precision), m, g);
+        e = local_launch(p, arith_of(ds.precision), m, g);
         if (e != cudaSuccess) return cuda_fail(e, "local-stage launch");
         if ((e = mark(1)) != cudaSuccess) return cuda_fail(e, "cudaEventRecord");
         if ((e = mark(2)) != cudaSuccess) return cuda_fail(e, "cudaEventRecord");
@@ -709,7 +767,7 @@ int solve_core(pbt_plan* p, double* a, double* b, double* c, double* d, int m, i
             if (ff && (e = pbt::launch_reduced_to_ff(p->rd, nsys, 2 * ds.nseg, m, p->status, s)) != cudaSuccess)
                 return cuda_fail(e, "reduced solution to float-float");
         } else {
-            e = cyclic ? run_reduced_cyclic(arith_of(ds.precision), m, g2) : run_reduced(arith_of(ds.precision), m, g2);
+            e = cyclic ? run_reduced_cyclic(arith_of(ds.precision), m, g2) : reduced_launch(p, arith_of(ds.precision), m, g2);
             if (e != cudaSuccess) return cuda_fail(e, "reduced-stage launch");
         }
         if ((e = mark(3)) != cudaSuccess) return cuda_fail(e, "cudaEventRecord");
@@ -949,7 +1007,10 @@ int pbt_solve_noncyclic_lines(pbt_plan* p, double* a, double* b, double* c, doub
                     "solve_lines: the lines span more than the plan's factor workspace (nsys*nrow*m*m); "
                     "use a PBT_FLAG_INPLACE plan for a non-dense layout");
     p->last_stream = s;
-    cudaError_t e = run_thomas_lines(arith_of(ds.precision), ds.m, make_args(p, a, b, c, d, s, ds.nsys), ls);
+    const int arith = arith_of(ds.precision);
+    const pbt::SolveArgs g = make_args(p, a, b, c, d, s, ds.nsys);
+    cudaError_t e = thomas_cols(p, arith, ds.m) ? run_thomas_cols(arith, ds.m, g, ls)
+                                                : run_thomas_lines(arith, ds.m, g, ls);
     if (e != cudaSuccess) return cuda_fail(e, "block Thomas launch (strided lines)");
     return PBT_OK;
 }
@@ -1044,8 +1105,8 @@ int pbt_adjoint_noncyclic(pbt_plan* p, const double* a, const double* b, const d
         if (e != cudaSuccess) return cuda_fail(e, "adjoint: transposed solve launch");
     } else {
         pbt::SolveArgs gs = make_args(p, p->at, p->bt, p->ct, g, s, ds.nsys * ds.nseg);
-        if ((e = run_modi(arith, m, gs)) != cudaSuccess ||
-            (e = run_reduced(arith, m, make_args(p, p->at, p->bt, p->ct, g, s, ds.nsys))) != cudaSuccess ||
+        if ((e = local_launch(p, arith, m, gs)) != cudaSuccess ||
+            (e = reduced_launch(p, arith, m, make_args(p, p->at, p->bt, p->ct, g, s, ds.nsys))) != cudaSuccess ||
             (e = run_update(arith, m, gs)) != cudaSuccess)
             return cuda_fail(e, "adjoint: transposed solve launch");
     }

@@ -16,6 +16,7 @@
 #endif
 #if defined(PBT_NUM_IS_F64) || defined(PBT_NUM_IS_FF)
 #include "pbt_batch.cuh"
+#include "pbt_cols.cuh"
 #endif
 
 namespace pbt {
@@ -32,6 +33,9 @@ template cudaError_t launch_update<PBT_NUM, PBT_M>(const SolveArgs&);
 template cudaError_t launch_adjoint<PBT_NUM, PBT_M>(const SolveArgs&, const AdjointArgs&);
 #if defined(PBT_NUM_IS_F64) || defined(PBT_NUM_IS_FF)
 template cudaError_t launch_batch<PBT_NUM, PBT_M>(const BatchArgs&, int, cudaStream_t, int*);
+template cudaError_t launch_thomas_cols<PBT_NUM, PBT_M>(const SolveArgs&, const LineStrides&);
+template cudaError_t launch_modi_cols<PBT_NUM, PBT_M>(const SolveArgs&);
+template cudaError_t launch_reduced_cols<PBT_NUM, PBT_M>(const SolveArgs&);
 #endif
 #ifdef PBT_NUM_IS_F64
 template cudaError_t launch_transpose_blocks<PBT_M>(const SolveArgs&, double*, double*, double*);

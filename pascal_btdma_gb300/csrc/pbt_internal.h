@@ -84,6 +84,13 @@ template <class Num, int M> cudaError_t launch_modi(const SolveArgs& g);
 template <class Num, int M> cudaError_t launch_reduced(const SolveArgs& g);
 template <class Num, int M> cudaError_t launch_reduced_cyclic(const SolveArgs& g);
 template <class Num, int M> cudaError_t launch_update(const SolveArgs& g);
+// One lane per block column (pbt_cols.cuh; F64 and FF, m <= kColsMaxBlock),
+// for batches too small for one thread per system: the single-segment solve of
+// lines by strides, the local stage, and the reduced solve.
+constexpr int kColsMaxBlock = PBT_MAX_BLOCK;
+template <class Num, int M> cudaError_t launch_thomas_cols(const SolveArgs& g, const LineStrides& ls);
+template <class Num, int M> cudaError_t launch_modi_cols(const SolveArgs& g);
+template <class Num, int M> cudaError_t launch_reduced_cols(const SolveArgs& g);
 // Adjoint (pbt_kernels.cuh: k_adjoint, k_transpose_blocks, k_gradients).
 struct AdjointArgs {
     const double* x;  // forward solution

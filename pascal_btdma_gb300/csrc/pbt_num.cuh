@@ -16,6 +16,7 @@
 //   T            register value;  Acc: an accumulator for sums of products
 //   in(p)        load an FP64 matrix element (A, B, C) and convert to T
 //   in_rhs(p)    the same for a right-hand-side element (D)
+//   in_value(v, rhs)  either, from a register (F64 and FF)
 //   out(p, v)    convert T to FP64 and store (f64(v): the converted value)
 //   lds/sts      raw 8-byte workspace slots (no conversion); from_raw: a slot's
 //                8 bytes already in a register
@@ -65,6 +66,7 @@ struct F64 {
     __device__ static __forceinline__ T in(const double* p) { return *p; }
     __device__ static __forceinline__ T in_ro(const double* p) { return __ldg(p); }
     __device__ static __forceinline__ T in_rhs(const double* p) { return *p; }
+    __device__ static __forceinline__ T in_value(double v, bool) { return v; }
     __device__ static __forceinline__ void out(double* p, T v) { *p = v; }
     __device__ static __forceinline__ double f64(T v) { return v; }
     __device__ static __forceinline__ T lds(const double* p) { return *p; }
@@ -135,7 +137,7 @@ struct FF {
     // every later operation carries into the solution, where the output check
     // (nonfinite) reports it: an input the arithmetic cannot carry gives a
     // reported failure, never a silently wrong number.
-    __device__ static __forceinline__ T split(double x) { return split_range<kFFExpLo, kFFExpHi, 1u>(x); }
+    __device__ static __forceinline__ T split(double x) { return split_range(x, kFFExpLo, kFFExpHi, 1u); }
     // The same conversion without the window, for right-hand sides and the
     // library's own intermediates (the reduced rows of a segmented plan after
     // an FP64 sub-solve, a refinement residual): |x| < 2^-126 gives 0,
@@ -145,20 +147,19 @@ struct FF {
     // diagonal blocks, or as the correction of a converged iterate; a whole
     // solution that small is caught by the output check, and an overflow is a
     // NaN in the solution.
-    __device__ static __forceinline__ T split_wide(double x) { return split_range<897u, 1150u, 897u>(x); }
-    // Biased FP64 exponents Lo..Hi convert, those below Zero give 0, the rest
-    // NaN.  14 instructions (18 with the low word cut out by shifts, 23 bits
-    // of it, and an exponent window on the shifted field), 80 of these a row
-    // at m = 5.
-    template <unsigned Lo, unsigned Hi, unsigned Zero>
-    __device__ static __forceinline__ T split_range(double x) {
+    __device__ static __forceinline__ T split_wide(double x) { return split_range(x, 897u, 1150u, 897u); }
+    // Biased FP64 exponents lo_e..hi_e convert, those below zero_e give 0, the
+    // rest NaN.  14 instructions (18 with the low word cut out by shifts, 23
+    // bits of it, and an exponent window on the shifted field), 80 of these a
+    // row at m = 5.
+    __device__ static __forceinline__ T split_range(double x, unsigned lo_e, unsigned hi_e, unsigned zero_e) {
         const unsigned hi = static_cast<unsigned>(__double2hiint(x));
         const unsigned lo = static_cast<unsigned>(__double2loint(x));
         const unsigned mag2 = hi << 1;  // exponent and the upper mantissa, without the sign
         // Rebias the exponent (1023 -> 127) and keep 23 mantissa bits; the sign back on top.
         const unsigned hb = (__funnelshift_l(lo, hi - (896u << 20), 3) & 0x7fffffffu) | (hi & 0x80000000u);
-        unsigned h = (mag2 - (Lo << 21) < ((Hi - Lo + 1u) << 21)) ? hb : 0x7fc00000u;
-        h = (mag2 < (Zero << 21)) ? 0u : h;
+        unsigned h = (mag2 - (lo_e << 21) < ((hi_e - lo_e + 1u) << 21)) ? hb : 0x7fc00000u;
+        h = (mag2 < (zero_e << 21)) ? 0u : h;
         // Sign and power of two of h (0 for zero, Inf for NaN) times the bits below it.
         const float l = __fmul_rn(__uint2float_rn(lo & 0x1fffffffu), __uint_as_float(h & 0xff800000u));
         return {__uint_as_float(h), __fmul_rn(l, 0x1p-52f)};
@@ -187,6 +188,11 @@ struct FF {
     __device__ static __forceinline__ T in(const double* p) { return split(*p); }
     __device__ static __forceinline__ T in_ro(const double* p) { return split(__ldg(p)); }
     __device__ static __forceinline__ T in_rhs(const double* p) { return split_wide(*p); }
+    // An input already in a register: a matrix element, or with `rhs` (which
+    // may differ between lanes) a right-hand-side element.
+    __device__ static __forceinline__ T in_value(double v, bool rhs) {
+        return split_range(v, rhs ? 897u : kFFExpLo, rhs ? 1150u : kFFExpHi, rhs ? 897u : 1u);
+    }
     __device__ static __forceinline__ void out(double* p, T v) { *p = join(v); }
     __device__ static __forceinline__ double f64(T v) { return join(v); }
     __device__ static __forceinline__ T lds(const double* p) {
