@@ -2666,7 +2666,7 @@ PBT_UNROLL
                     for (int k = 0; k < M; ++k) {
                         const double a = __ldg(g.a + sys + o + (size_t)(i + M * k) * plane);
                         r[i] = fma(-a, xm[k], r[i]);
-                        an[i][k] = FF::split(a).h;
+                        an[i][k] = F32::narrow(a);
                     }
             }
             if (has_next) {
@@ -2677,7 +2677,7 @@ PBT_UNROLL
                         r[i] = fma(-__ldg(g.c + sys + o + (size_t)(i + M * k) * plane), xp[k], r[i]);
             }
 PBT_UNROLL
-            for (int i = 0; i < M; ++i) ta[i] = F32::acc(FF::split_wide(r[i]).h);
+            for (int i = 0; i < M; ++i) ta[i] = F32::acc(F32::narrow_wide(r[i]));
             if (q > 0) {
 PBT_UNROLL
                 for (int k = 0; k < M; ++k)

@@ -276,9 +276,21 @@ struct F32 {
     // more than the solve itself.  Matrix entries take float-float's window
     // (a row scaled out of it cannot be refined: its residuals fall below
     // FP32's range); right-hand sides and residuals convert without it.
-    __device__ static __forceinline__ T in(const double* p) { return FF::split(*p).h; }
-    __device__ static __forceinline__ T in_ro(const double* p) { return FF::split(__ldg(p)).h; }
-    __device__ static __forceinline__ T in_rhs(const double* p) { return FF::split_wide(*p).h; }
+    // The high word of FF::split / FF::split_wide from the exponent field
+    // alone, which schedules better without the low word (refined solve,
+    // m = 5, 65536 x 256: 6436 us against 6456 with theirs).
+    __device__ static __forceinline__ T high(double x, unsigned lo_e, unsigned hi_e, unsigned zero_e) {
+        const unsigned hi = static_cast<unsigned>(__double2hiint(x));
+        const unsigned lo = static_cast<unsigned>(__double2loint(x));
+        const unsigned e = (hi >> 20) & 0x7ffu;
+        const unsigned hb = __funnelshift_l(lo, (hi & 0x7fffffffu) - (896u << 20), 3) | (hi & 0x80000000u);
+        return __uint_as_float(e - lo_e <= hi_e - lo_e ? hb : (e >= zero_e ? 0x7fc00000u : 0u));
+    }
+    __device__ static __forceinline__ T narrow(double x) { return high(x, kFFExpLo, kFFExpHi, 1u); }
+    __device__ static __forceinline__ T narrow_wide(double x) { return high(x, 897u, 1150u, 897u); }
+    __device__ static __forceinline__ T in(const double* p) { return narrow(*p); }
+    __device__ static __forceinline__ T in_ro(const double* p) { return narrow(__ldg(p)); }
+    __device__ static __forceinline__ T in_rhs(const double* p) { return narrow_wide(*p); }
     __device__ static __forceinline__ void out(double* p, T v) { *p = FF::widen(v); }
     __device__ static __forceinline__ double f64(T v) { return FF::widen(v); }
     // Raw slots are written whole (the float and a zero pad), so every 32-byte

@@ -571,7 +571,7 @@ PBT_UNROLL
             for (int i = 0; i < M; ++i) {
                 const double a = p[32 * i];
                 if (q > 0) r[i] = fma(-a, xm[k], r[i]);
-                an[i][k] = FF::split(a).h;
+                an[i][k] = F32::narrow(a);
             }
             give();
         }
@@ -587,7 +587,7 @@ PBT_UNROLL
         if (!ok) break;
         F32::Acc ta[M];
 PBT_UNROLL
-        for (int i = 0; i < M; ++i) ta[i] = F32::acc(FF::split_wide(r[i]).h);
+        for (int i = 0; i < M; ++i) ta[i] = F32::acc(F32::narrow_wide(r[i]));
         if (q > 0) {
 PBT_UNROLL
             for (int k = 0; k < M; ++k)
