@@ -32,8 +32,8 @@ struct pbt_batch {
     int2* items3 = nullptr;
     long long* d_user_mat_off = nullptr;
     long long* d_user_vec_off = nullptr;
-    long long* row_start = nullptr;
-    long long pack_total = 0;
+    int* chunk_start = nullptr;
+    int pack_chunks = 0;
     int* state = nullptr;  // error (always 0), pad, head1[m] (kHeads), seg_done[ntiles]
     unsigned long long* status = nullptr;
     double *aw = nullptr, *cw = nullptr, *ra = nullptr, *rc = nullptr, *rd = nullptr;
@@ -106,7 +106,7 @@ void free_batch(pbt_batch* b) {
     cudaFree(b->items3);
     cudaFree(b->d_user_mat_off);
     cudaFree(b->d_user_vec_off);
-    cudaFree(b->row_start);
+    cudaFree(b->chunk_start);
     cudaFree(b->state);
     cudaFree(b->status);
     cudaFree(b->aw);
@@ -177,8 +177,8 @@ int pbt_batch_create(pbt_batch** out, int nsys, const int* m, const int* nrow, i
     });
     std::vector<pbt::BatchTile> tiles;
     std::vector<int> lane_rows, sys_of;
-    std::vector<long long> row_start;
-    long long mat_off = 0, vec_off = 0, red_m = 0, red_v = 0, rowacc = 0;
+    std::vector<int> chunk_start;
+    long long mat_off = 0, vec_off = 0, red_m = 0, red_v = 0, chunks = 0;
     for (int k = 0; k < nsys;) {
         const int mm = m[order[k]];
         int lanes = 0;
@@ -206,8 +206,8 @@ int pbt_batch_create(pbt_batch** out, int nsys, const int* m, const int* nrow, i
             red_m += 32LL * 2 * P * mm * mm;
             red_v += 32LL * 2 * P * mm;
         }
-        row_start.push_back(rowacc);
-        rowacc += 32LL * t.rows;
+        chunk_start.push_back((int)chunks);
+        chunks += (t.rows + pbt::kPackRows - 1) / pbt::kPackRows;
         for (int l = 0; l < 32; ++l) {
             lane_rows.push_back(l < lanes ? nrow[order[k + l]] : 0);
             sys_of.push_back(l < lanes ? order[k + l] : -1);
@@ -220,7 +220,7 @@ int pbt_batch_create(pbt_batch** out, int nsys, const int* m, const int* nrow, i
     b->packed_vec = vec_off;
     b->red_mat = red_m;
     b->red_vec = red_v;
-    b->pack_total = rowacc;
+    b->pack_chunks = (int)chunks;  // fits: the packed arrays take at least 512 bytes a chunk
     // Work items, per block size.  Stage 1 by decreasing cost (m^3 * rows of
     // the item; the two-stage elimination costs ~2.4x block Thomas per row);
     // stage 3 in the order stage 1 first reaches each tile.  The launches run
@@ -273,7 +273,7 @@ int pbt_batch_create(pbt_batch** out, int nsys, const int* m, const int* nrow, i
     if ((rc = upload(&b->tiles, tiles)) || (rc = upload(&b->lane_rows, lane_rows)) || (rc = upload(&b->sys_of, sys_of)) ||
         (rc = upload(&b->items1, items1)) || (rc = upload(&b->items3, items3)) ||
         (rc = upload(&b->d_user_mat_off, b->user_mat_off)) || (rc = upload(&b->d_user_vec_off, b->user_vec_off)) ||
-        (rc = upload(&b->row_start, row_start)))
+        (rc = upload(&b->chunk_start, chunk_start)))
         goto fail_out;
     {
         cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&b->state), sizeof(int) * state_ints(b->ntiles));
@@ -332,9 +332,9 @@ static pbt::PackArgs pack_args(const pbt_batch* b) {
     pa.sys_of = b->sys_of;
     pa.user_mat_off = b->d_user_mat_off;
     pa.user_vec_off = b->d_user_vec_off;
-    pa.row_start = b->row_start;
+    pa.chunk_start = b->chunk_start;
     pa.ntiles = b->ntiles;
-    pa.total = b->pack_total;
+    pa.chunks = b->pack_chunks;
     return pa;
 }
 

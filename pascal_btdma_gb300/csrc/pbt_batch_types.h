@@ -45,10 +45,11 @@ struct PackArgs {
     const int* sys_of;              // [tile*32 + lane]: system index, -1 = empty lane
     const long long* user_mat_off;  // per system
     const long long* user_vec_off;
-    const long long* row_start;     // per tile: prefix sum of 32*rows
+    const int* chunk_start;         // per tile: prefix sum of its chunks of kPackRows rows
     int ntiles;
-    long long total;                // sum over tiles of 32*rows
+    int chunks;                     // of all tiles
 };
+constexpr int kPackRows = 64;
 
 // The launches of block size M (pbt_batch.cuh; instantiated with the other
 // kernels of (Num, M) in pbt_inst.cu).
