@@ -281,8 +281,9 @@ bool encode_columns_f32(CUtensorMap* tm, const double* base, int nsys, int nrow,
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Launch the single-segment block Thomas solve, with TMA-staged loads
-// (k_thomas_staged) or direct loads (k_thomas); both give the same bits.
+// With neither column lanes (cols_pay) nor the CTA's ring (prefer_ring): the
+// single-segment block Thomas solve with TMA-staged loads (k_thomas_staged) or
+// direct loads (k_thomas); all give the same bits.
 // The default follows GB300 measurements (float-float unless noted, N = 256
 // or 512): staged loads win for the FP32 factorisation of the refined solve,
 // which is bound by memory (m = 5, 65536 systems: 11.5 vs 12.2 ms); for
@@ -364,9 +365,77 @@ bool thomas_cols(const pbt_plan* p, int arith, int m) {
            cols_pay(arith, m, p->desc.nsys, false, p->sms);
 }
 
+// The same for lines by strides: dimensions {lines along the fast index, rows
+// and outer lines (the smaller stride first), planes}, boxes of one block
+// column of 32 lines.  *row_first: the rows come before the outer lines.
+bool encode_lines(CUtensorMap* tm, const double* base, int nsys, int nrow, const pbt::LineStrides& ls, int planes, int m,
+                  int* row_first) {
+    const PFN_cuTensorMapEncodeTiled_v12000 fn = tensor_map_encoder();
+    if (fn == nullptr || base == nullptr || (reinterpret_cast<std::uintptr_t>(base) & 15u) != 0) return false;
+    const int outer = nsys / ls.lin;
+    if (ls.in != 1 || ((ls.row | ls.elem | ls.out) & 1) || ls.row <= 0 || ls.elem <= 0) return false;
+    if (outer > 1 && (ls.lin % 32 != 0 || ls.out <= 0)) return false;
+    const cuuint64_t so = outer > 1 ? (cuuint64_t)ls.out : (cuuint64_t)ls.row * (cuuint64_t)nrow;
+    const bool rf = (cuuint64_t)ls.row <= so;
+    *row_first = rf ? 1 : 0;
+    const cuuint64_t dims[4] = {(cuuint64_t)ls.lin, (cuuint64_t)(rf ? nrow : outer), (cuuint64_t)(rf ? outer : nrow),
+                                (cuuint64_t)planes};
+    const cuuint64_t strides[3] = {8u * (rf ? (cuuint64_t)ls.row : so), 8u * (rf ? so : (cuuint64_t)ls.row),
+                                   8u * (cuuint64_t)ls.elem};
+    const cuuint32_t box[4] = {32u, 1u, 1u, (cuuint32_t)m};
+    const cuuint32_t estr[4] = {1u, 1u, 1u, 1u};
+    return fn(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, const_cast<double*>(base), dims, strides, box, estr,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// Whether the single-segment solve of a batch past cols_pay's line runs through
+// the CTA's ring (pbt_ring.cuh), from sweeps over 11000 to 131072 systems
+// (GB300; us, without -> with): float-float m = 3, 4 (28000 x 64, m = 4 619 ->
+// 529; 100000 883 -> 667 and 1523 -> 1250); FP64 m = 4 .. 6 (m = 5 11000 x 64
+// 1287 -> 1180, 65536 3177 -> 3080, 100000 5179 -> 4634), except m = 5, 6
+// between 180 and 256 threads an SM, where k_thomas_staged's one-warp CTAs
+// spread better (32768 1650 against 1712); FP64 m = 3 from 400 threads an SM on
+// (40960 668 against 692, 100000 1488 -> 1369).  m <= 2 was not tried: too few
+// values an item.
+bool prefer_ring(int arith, int m, int nsys, int sms) {
+    const long long per = nsys / (sms > 0 ? sms : 1);
+    if (arith == kFF) return m == 3 || m == 4;
+    if (arith != kF64) return false;
+    return m == 3 ? per >= 400 : m == 4 || ((m == 5 || m == 6) && !(per >= 180 && per < 256));
+}
+// Launches it if the rule and the tensor maps allow; false: not launched.
+bool ring_launch(const pbt_plan* p, int arith, int m, const pbt::SolveArgs& g, const pbt::LineStrides& ls,
+                 cudaError_t* e) {
+    if (!g.tpb_auto || (p->desc.flags & (PBT_FLAG_DIRECT_LOADS | PBT_FLAG_STAGED_LOADS)) ||
+        !prefer_ring(arith, m, g.nsys, p->sms))
+        return false;
+    const int mm = m * m;
+    pbt::ThomasMaps maps;
+    int rf = 0;
+    if (!encode_lines(&maps.a, g.a, g.nsys, g.nrow, ls, mm, m, &rf) ||
+        !encode_lines(&maps.b, g.b, g.nsys, g.nrow, ls, mm, m, &rf) ||
+        !encode_lines(&maps.c, g.c, g.nsys, g.nrow, ls, mm, m, &rf) ||
+        !encode_lines(&maps.d, g.d, g.nsys, g.nrow, ls, m, m, &rf) ||
+        !encode_lines(&maps.w, g.cw, g.nsys, g.nrow, ls, mm, m, &rf))
+        return false;
+    if (arith == kFF)
+        *e = m == 3 ? pbt::launch_thomas_ring<pbt::FF, 3>(g, ls, maps, rf) : pbt::launch_thomas_ring<pbt::FF, 4>(g, ls, maps, rf);
+    else
+        switch (m) {
+            case 3: *e = pbt::launch_thomas_ring<pbt::F64, 3>(g, ls, maps, rf); break;
+            case 4: *e = pbt::launch_thomas_ring<pbt::F64, 4>(g, ls, maps, rf); break;
+            case 5: *e = pbt::launch_thomas_ring<pbt::F64, 5>(g, ls, maps, rf); break;
+            default: *e = pbt::launch_thomas_ring<pbt::F64, 6>(g, ls, maps, rf); break;
+        }
+    return *e != cudaErrorNotSupported;
+}
+
 cudaError_t thomas_launch(const pbt_plan* p, int arith, int m, const pbt::SolveArgs& g) {
-    if (thomas_cols(p, arith, m))
-        return run_thomas_cols(arith, m, g, {g.nsys, 1, 0, g.nsys, (long long)g.nsys * g.nrow});
+    const pbt::LineStrides plain{g.nsys, 1, 0, g.nsys, (long long)g.nsys * g.nrow};
+    if (thomas_cols(p, arith, m)) return run_thomas_cols(arith, m, g, plain);
+    cudaError_t e;
+    if (ring_launch(p, arith, m, g, plain, &e)) return e;
     pbt::ThomasMaps maps;
     return thomas_stages(p, arith, m, g, &maps) ? run_thomas_staged(arith, m, g, maps) : run_thomas(arith, m, g);
 }
@@ -1009,8 +1078,11 @@ int pbt_solve_noncyclic_lines(pbt_plan* p, double* a, double* b, double* c, doub
     p->last_stream = s;
     const int arith = arith_of(ds.precision);
     const pbt::SolveArgs g = make_args(p, a, b, c, d, s, ds.nsys);
-    cudaError_t e = thomas_cols(p, arith, ds.m) ? run_thomas_cols(arith, ds.m, g, ls)
-                                                : run_thomas_lines(arith, ds.m, g, ls);
+    cudaError_t e;
+    if (thomas_cols(p, arith, ds.m))
+        e = run_thomas_cols(arith, ds.m, g, ls);
+    else if (!ring_launch(p, arith, ds.m, g, ls, &e))
+        e = run_thomas_lines(arith, ds.m, g, ls);
     if (e != cudaSuccess) return cuda_fail(e, "block Thomas launch (strided lines)");
     return PBT_OK;
 }

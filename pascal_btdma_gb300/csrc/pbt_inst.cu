@@ -18,6 +18,10 @@
 #include "pbt_batch.cuh"
 #include "pbt_cols.cuh"
 #endif
+#if PBT_M >= 3 && ((defined(PBT_NUM_IS_F64) && PBT_M <= 6) || (defined(PBT_NUM_IS_FF) && PBT_M <= 4))
+#include "pbt_ring.cuh"
+#define PBT_HAS_RING
+#endif
 
 namespace pbt {
 template cudaError_t launch_thomas<PBT_NUM, PBT_M>(const SolveArgs&);
@@ -36,6 +40,9 @@ template cudaError_t launch_batch<PBT_NUM, PBT_M>(const BatchArgs&, int, cudaStr
 template cudaError_t launch_thomas_cols<PBT_NUM, PBT_M>(const SolveArgs&, const LineStrides&);
 template cudaError_t launch_modi_cols<PBT_NUM, PBT_M>(const SolveArgs&);
 template cudaError_t launch_reduced_cols<PBT_NUM, PBT_M>(const SolveArgs&);
+#endif
+#ifdef PBT_HAS_RING
+template cudaError_t launch_thomas_ring<PBT_NUM, PBT_M>(const SolveArgs&, const LineStrides&, const ThomasMaps&, int);
 #endif
 #ifdef PBT_NUM_IS_F64
 template cudaError_t launch_transpose_blocks<PBT_M>(const SolveArgs&, double*, double*, double*);

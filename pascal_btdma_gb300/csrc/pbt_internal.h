@@ -77,6 +77,10 @@ template <class Num, int M> cudaError_t launch_thomas_lines(const SolveArgs& g, 
 cudaError_t launch_lines_layout(const double* src, double* dst, const LineStrides& ls, int E, int nsys, int nrow,
                                 int dir, cudaStream_t s);
 template <class Num, int M> cudaError_t launch_thomas_staged(const SolveArgs& g, const ThomasMaps& maps);
+// The solve through a CTA-wide ring (pbt_ring.cuh), maps over {lines, rows and
+// outer lines, planes}; cudaErrorNotSupported where its shared memory does not fit.
+template <class Num, int M>
+cudaError_t launch_thomas_ring(const SolveArgs& g, const LineStrides& ls, const ThomasMaps& maps, int row_first);
 // Periodic lines in one segment (k_thomas_cyclic): the fill-in column in
 // g.re, nsys * nrow * m * m raw values; nrow >= 3.
 template <class Num, int M> cudaError_t launch_thomas_cyclic(const SolveArgs& g);
