@@ -157,7 +157,9 @@ void pbt_plan_desc_init(pbt_plan_desc* desc);
  * the GPU with one thread per system (nsys >= 128 * SMs, 19456 on a GB300)
  * is solved one segment per line whatever nseg says: the single-segment
  * method does ~40 % of the two-stage method's arithmetic and gives the same x
- * to rounding.  PBT_FLAG_REFERENCE_METHOD keeps the nseg segments (and the
+ * to rounding.  Non-cyclic FP64 and PBT_PREC_FF plans that are not in place do
+ * so from m = 3 and fewer systems on, where that is faster (8 to 78 * SMs by m and
+ * precision).  PBT_FLAG_REFERENCE_METHOD keeps the nseg segments (and the
  * reference's in-place A', C' with PBT_FLAG_INPLACE). */
 int pbt_plan_create(pbt_plan** plan, int m, int nsys, int nrow, int nseg);
 

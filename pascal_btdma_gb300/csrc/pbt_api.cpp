@@ -47,6 +47,7 @@ struct pbt_plan {
     int device = 0;
     int sms = 0;          // multiprocessors of `device`
     bool thomas = false;  // single-segment plain block Thomas path
+    bool lines = false;   // strided lines and the fused adjoint: nseg = 1, or a batch that fills the GPU
     bool cyclic_thomas = false;  // single-segment periodic block Thomas (k_thomas_cyclic)
     double* aw = nullptr;  // factor workspace (nullptr when in place)
     double* cw = nullptr;
@@ -492,6 +493,33 @@ bool fills_gpu(int nsys, int sms) {
     return warps >= 4LL * (sms > 0 ? sms : 152);
 }
 
+// Whether a smaller batch, too, is better solved one segment per line than in
+// its nseg > 1 segments: from so many systems that the line's chain of rows,
+// with one lane per block column (pbt_cols.cuh), takes no longer than the
+// two-stage method's 2.4 times the arithmetic (systems an SM; GB300, us,
+// segments -> one segment):
+//   float-float m = 3, 12347 x 301 in 3 897 -> 709, 3000 x 512 in 16 513 -> 627
+//     (line at 30); m = 5, 2500 x 512 in 16 1598 -> 1201, 1500 984 -> 1100 (14);
+//     m = 6, 1300 2161 -> 1894, 900 1594 -> 1862 (8); m = 8, 1600 3691 -> 3352,
+//     1000 2385 -> 3306 (9);
+//   FP64, whose pipe the local stage fills with fewer warps: m = 3, 4000 x 512
+//     in 16 1459 -> 1228 (22; 1024 x 128 in 4 150 -> 301); m = 4, 12000 5743 ->
+//     5409, 8000 4401 -> 4547 (78); m = 5, 3000 2872 -> 2840, 2000 2283 -> 2677
+//     (18); m = 8, 1300 6550 -> 6401, 800 5031 -> 6323, 4096 x 1024 in 4 39237
+//     -> 30475 (8).
+// m <= 2 keeps its segments up to fills_gpu's line (FP64 m = 2, 14000 x 512 in
+// 16 1222 -> 1686; float-float 13000 626 -> 628).
+// Not for plans whose factors the caller gets (in place) or that ask for the
+// reference method.
+bool one_segment_pays(const pbt_plan_desc& d, int sms) {
+    if (d.precision == PBT_PREC_FP32_REFINE ||
+        (d.flags & (PBT_FLAG_CYCLIC | PBT_FLAG_INPLACE | PBT_FLAG_REFERENCE_METHOD)))
+        return false;
+    static const int ff[] = {128, 128, 30, 30, 14, 8, 11, 9}, fp64[] = {128, 128, 22, 78, 18, 13, 11, 8};
+    const int line = (d.precision == PBT_PREC_FF ? ff : fp64)[d.m < 8 ? d.m - 1 : 7];
+    return d.nsys >= line * (long long)(sms > 0 ? sms : 152);
+}
+
 // The local-stage and update launches put the segments in gridDim.y.
 constexpr int kMaxSegments = 65535;
 
@@ -898,13 +926,15 @@ int pbt_plan_create_ex(pbt_plan** out, const pbt_plan_desc* desc) {
     const bool inplace = (d.flags & PBT_FLAG_INPLACE) != 0;
     const bool cyclic = (d.flags & PBT_FLAG_CYCLIC) != 0;
     // nseg is the reference's decomposition of a line over MPI ranks.  On one
-    // GPU, a batch with enough systems to fill it is solved one segment per
-    // line (the method of nseg = 1: ~40 % of the two-stage method's
-    // arithmetic, same x to rounding) unless PBT_FLAG_REFERENCE_METHOD asks for
-    // the segments.
-    const bool one_seg = d.nseg == 1 || (!(d.flags & PBT_FLAG_REFERENCE_METHOD) && fills_gpu(d.nsys, p->sms) &&
-                                         (!cyclic || d.nrow >= 3));
+    // GPU, a batch with enough systems (fills_gpu, one_segment_pays) is solved
+    // one segment per line (the method of nseg = 1: ~40 % of the two-stage
+    // method's arithmetic, same x to rounding) unless
+    // PBT_FLAG_REFERENCE_METHOD asks for the segments.
+    const bool full = d.nseg == 1 || (!(d.flags & PBT_FLAG_REFERENCE_METHOD) && fills_gpu(d.nsys, p->sms) &&
+                                      (!cyclic || d.nrow >= 3));
+    const bool one_seg = full || one_segment_pays(d, p->sms);
     p->thomas = one_seg && !cyclic && !(d.flags & PBT_FLAG_REFERENCE_METHOD);
+    p->lines = p->thomas && full;
     p->cyclic_thomas = one_seg && cyclic;
     const size_t mm = (size_t)d.m * d.m;
     const size_t rows = (size_t)d.nsys * d.nrow;
@@ -1019,7 +1049,7 @@ int pbt_solve_noncyclic_lines(pbt_plan* p, double* a, double* b, double* c, doub
     if (rc) return rc;
     const pbt_plan_desc& ds = p->desc;
     if (!a || !b || !c || !d || !L) return fail(PBT_EINVAL, "solve_lines: null argument");
-    if (!p->thomas || (ds.flags & PBT_FLAG_CPU_LAYOUT) || ds.precision == PBT_PREC_FP32_REFINE)
+    if (!p->lines || (ds.flags & PBT_FLAG_CPU_LAYOUT) || ds.precision == PBT_PREC_FP32_REFINE)
         return fail(PBT_EUNSUPPORTED,
                     "solve_lines: needs a single-segment, non-cyclic FP64 or float-float plan in the GPU layout");
     if (L->nsys_inner <= 0 || L->nsys_outer <= 0 || (long long)L->nsys_inner * L->nsys_outer != ds.nsys) {
@@ -1156,13 +1186,13 @@ int pbt_adjoint_noncyclic(pbt_plan* p, const double* a, const double* b, const d
     adj.dc = dc;
     const int arith = arith_of(ds.precision);
     cudaError_t e;
-    if (p->thomas) {
+    if (p->lines) {
         e = run_adjoint(arith, m, make_args(p, const_cast<double*>(a), const_cast<double*>(b),
                                             const_cast<double*>(c), g, s, ds.nsys), adj);
         if (e != cudaSuccess) return cuda_fail(e, "adjoint launch");
         return PBT_OK;
     }
-    // Segmented plans: materialise M^T and solve it with the plan's own
+    // Plans of nseg > 1: materialise M^T and solve it with the plan's own
     // forward method.
     if (!p->at) {
         const size_t n = (size_t)ds.m * ds.m * ds.nsys * ds.nrow;
