@@ -326,6 +326,12 @@ cudaError_t run_thomas_cols(int arith, int m, const pbt::SolveArgs& g, const pbt
     }
     PBT_DISPATCH_PLAIN_M2(pbt::F64, launch_thomas_cols, g, ls)
 }
+cudaError_t run_transposed_cols(int arith, int m, const pbt::SolveArgs& g) {
+    if (arith == kFF) {
+        PBT_DISPATCH_PLAIN_M2(pbt::FF, launch_transposed_cols, g)
+    }
+    PBT_DISPATCH_PLAIN_M2(pbt::F64, launch_transposed_cols, g)
+}
 cudaError_t run_modi_cols(int arith, int m, const pbt::SolveArgs& g) {
     if (arith == kFF) {
         PBT_DISPATCH_PLAIN_M2(pbt::FF, launch_modi_cols, g)
@@ -428,6 +434,54 @@ bool ring_launch(const pbt_plan* p, int arith, int m, const pbt::SolveArgs& g, c
             case 4: *e = pbt::launch_thomas_ring<pbt::F64, 4>(g, ls, maps, rf); break;
             case 5: *e = pbt::launch_thomas_ring<pbt::F64, 5>(g, ls, maps, rf); break;
             default: *e = pbt::launch_thomas_ring<pbt::F64, 6>(g, ls, maps, rf); break;
+        }
+    return *e != cudaErrorNotSupported;
+}
+
+// A block array as {nsys, nrow, 1, m, m}, boxes of one block row of 32 systems
+// (the transposed solve's columns).
+bool encode_block_rows(CUtensorMap* tm, const double* base, int nsys, int nrow, int m) {
+    const PFN_cuTensorMapEncodeTiled_v12000 fn = tensor_map_encoder();
+    if (fn == nullptr || base == nullptr || (reinterpret_cast<std::uintptr_t>(base) & 15u) != 0 || (nsys & 1))
+        return false;
+    const cuuint64_t plane = (cuuint64_t)nsys * (cuuint64_t)nrow * 8u;
+    const cuuint64_t dims[5] = {(cuuint64_t)nsys, (cuuint64_t)nrow, 1, (cuuint64_t)m, (cuuint64_t)m};
+    const cuuint64_t strides[4] = {(cuuint64_t)nsys * 8u, plane, plane, plane * (cuuint64_t)m};
+    const cuuint32_t box[5] = {32u, 1u, 1u, 1u, (cuuint32_t)m};
+    const cuuint32_t estr[5] = {1u, 1u, 1u, 1u, 1u};
+    return fn(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 5, const_cast<double*>(base), dims, strides, box, estr,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// M^T lambda = g (in g.d) of a single-segment plan, straight from the stored
+// blocks: by column lanes or through the ring where the forward solve takes
+// them; false: neither, not launched.
+bool transposed_launch(const pbt_plan* p, int arith, int m, const pbt::SolveArgs& g, cudaError_t* e) {
+    if (thomas_cols(p, arith, m)) {
+        *e = run_transposed_cols(arith, m, g);
+        return true;
+    }
+    if (!g.tpb_auto || (p->desc.flags & (PBT_FLAG_DIRECT_LOADS | PBT_FLAG_STAGED_LOADS)) ||
+        !prefer_ring(arith, m, g.nsys, p->sms))
+        return false;
+    const pbt::LineStrides ls{g.nsys, 1, 0, g.nsys, (long long)g.nsys * g.nrow};
+    const int mm = m * m;
+    pbt::ThomasMaps maps;
+    int rf = 0;
+    if (!encode_block_rows(&maps.a, g.c, g.nsys, g.nrow, m) || !encode_block_rows(&maps.b, g.b, g.nsys, g.nrow, m) ||
+        !encode_block_rows(&maps.c, g.a, g.nsys, g.nrow, m) ||
+        !encode_lines(&maps.d, g.d, g.nsys, g.nrow, ls, m, m, &rf) ||
+        !encode_lines(&maps.w, g.cw, g.nsys, g.nrow, ls, mm, m, &rf) || !rf)
+        return false;
+    if (arith == kFF)
+        *e = m == 3 ? pbt::launch_transposed_ring<pbt::FF, 3>(g, ls, maps) : pbt::launch_transposed_ring<pbt::FF, 4>(g, ls, maps);
+    else
+        switch (m) {
+            case 3: *e = pbt::launch_transposed_ring<pbt::F64, 3>(g, ls, maps); break;
+            case 4: *e = pbt::launch_transposed_ring<pbt::F64, 4>(g, ls, maps); break;
+            case 5: *e = pbt::launch_transposed_ring<pbt::F64, 5>(g, ls, maps); break;
+            default: *e = pbt::launch_transposed_ring<pbt::F64, 6>(g, ls, maps); break;
         }
     return *e != cudaErrorNotSupported;
 }
@@ -1186,9 +1240,21 @@ int pbt_adjoint_noncyclic(pbt_plan* p, const double* a, const double* b, const d
     adj.dc = dc;
     const int arith = arith_of(ds.precision);
     cudaError_t e;
+    const pbt::SolveArgs g0 = make_args(p, const_cast<double*>(a), const_cast<double*>(b), const_cast<double*>(c),
+                                        g, s, ds.nsys);
+    // Where the forward solve runs by column lanes or through the ring, the
+    // transposed one does too, and the gradient blocks, which are independent
+    // of each other, follow at HBM speed; else the fused kernel.  us, fused or
+    // through materialised transposes -> this: m = 4 16384 x 512 FP64 7104 ->
+    // 6427 (nseg = 8: 7598 -> 6438), float-float 5948 -> 3771; m = 4 1024 x 128
+    // FP64 1676 -> 535; m = 5 4096 x 128 float-float 2569 -> 538.
+    if (p->thomas && transposed_launch(p, arith, m, g0, &e)) {
+        if (e == cudaSuccess && (da || db || dc)) e = run_gradients(m, g0, adj);
+        if (e != cudaSuccess) return cuda_fail(e, "adjoint launch");
+        return PBT_OK;
+    }
     if (p->lines) {
-        e = run_adjoint(arith, m, make_args(p, const_cast<double*>(a), const_cast<double*>(b),
-                                            const_cast<double*>(c), g, s, ds.nsys), adj);
+        e = run_adjoint(arith, m, g0, adj);
         if (e != cudaSuccess) return cuda_fail(e, "adjoint launch");
         return PBT_OK;
     }
@@ -1198,8 +1264,6 @@ int pbt_adjoint_noncyclic(pbt_plan* p, const double* a, const double* b, const d
         const size_t n = (size_t)ds.m * ds.m * ds.nsys * ds.nrow;
         if ((rc = alloc(p, &p->at, n)) || (rc = alloc(p, &p->bt, n)) || (rc = alloc(p, &p->ct, n))) return rc;
     }
-    const pbt::SolveArgs g0 = make_args(p, const_cast<double*>(a), const_cast<double*>(b), const_cast<double*>(c),
-                                        g, s, ds.nsys);
     if ((e = run_transpose_blocks(m, g0, p->at, p->bt, p->ct)) != cudaSuccess)
         return cuda_fail(e, "adjoint: transpose launch");
     if (p->thomas) {

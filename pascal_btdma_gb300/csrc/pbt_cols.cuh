@@ -60,11 +60,11 @@ __device__ __forceinline__ ColLane col_lane(long long nsys) {
     return c;
 }
 
-// M values `plane` apart at p (zeros on a lane that is not live), raw.
+// M values `stride` apart at p (zeros on a lane that is not live), raw.
 template <int M>
-__device__ __forceinline__ void col_load(double (&v)[M], const double* p, size_t plane, bool live) {
+__device__ __forceinline__ void col_load(double (&v)[M], const double* p, size_t stride, bool live) {
 #pragma unroll
-    for (int i = 0; i < M; ++i) v[i] = live ? p[(size_t)i * plane] : 0.0;
+    for (int i = 0; i < M; ++i) v[i] = live ? p[(size_t)i * stride] : 0.0;
 }
 
 // One elimination of the group's R (lane j < M: column j in r; consumed) on NX
@@ -191,8 +191,9 @@ __host__ __device__ constexpr int cols_ahead() {
 
 // Single-segment block Thomas of one system per group.  Pointers at the
 // system's first row; Reduced: the reduced system of the two-stage method (B =
-// I, everything raw; A, C', d in RA, RC, RD).
-template <class Num, int M, bool Reduced>
+// I, everything raw; A, C', d in RA, RC, RD); Transposed: A, B and C hold the
+// transposed blocks (column j of a block is row j of what is stored).
+template <class Num, int M, bool Reduced, bool Transposed = false>
 __device__ __forceinline__ void thomas_cols_body(const double* A, const double* B, const double* C, double* D,
                                                  double* CW, size_t plane, size_t rs, int N, bool raw,
                                                  unsigned long long* status, const ColLane& cl) {
@@ -200,10 +201,12 @@ __device__ __forceinline__ void thomas_cols_body(const double* A, const double* 
     using Acc = typename Num::Acc;
     const bool rhs = cl.j == M;
     const size_t col = (size_t)(rhs ? 0 : cl.j) * M * plane;
+    const size_t in = Transposed ? (size_t)(rhs ? 0 : cl.j) * plane : col;  // this lane's column of an input block
+    const size_t es = Transposed ? M * plane : plane, eb = Transposed && !rhs ? es : plane;
     const bool mat = cl.live && !rhs;
-    const double* const pa = A + col;
-    const double* const pb = rhs ? D : (Reduced ? A : B + col);
-    const double* const pc = C + col;
+    const double* const pa = A + in;
+    const double* const pb = rhs ? D : (Reduced ? A : B + in);
+    const double* const pc = C + in;
     double* const pw = rhs ? D : CW + col;
     unsigned bad = 0, amax = 0;
     double va[M], vb[M], vc[M];
@@ -212,8 +215,8 @@ __device__ __forceinline__ void thomas_cols_body(const double* A, const double* 
     if constexpr (Reduced)
         col_load<M>(vb, pb, plane, cl.live && rhs);
     else
-        col_load<M>(vb, pb, plane, cl.live);
-    col_load<M>(vc, pc, plane, mat && N > 1);
+        col_load<M>(vb, pb, eb, cl.live);
+    col_load<M>(vc, pc, es, mat && N > 1);
     for (int q = 0; q < N; ++q) {
         const size_t o = (size_t)q * rs;
         const bool last = q == N - 1;
@@ -231,12 +234,12 @@ __device__ __forceinline__ void thomas_cols_body(const double* A, const double* 
         // The next row's inputs, on their way while this row is eliminated.
         if (!last) {
             const size_t p = o + rs;
-            col_load<M>(va, pa + p, plane, mat);
+            col_load<M>(va, pa + p, es, mat);
             if constexpr (Reduced)
                 col_load<M>(vb, pb + p, plane, cl.live && rhs);
             else
-                col_load<M>(vb, pb + p, plane, cl.live);
-            col_load<M>(vc, pc + p, plane, mat && q + 2 < N);
+                col_load<M>(vb, pb + p, eb, cl.live);
+            col_load<M>(vc, pc + p, es, mat && q + 2 < N);
         }
         if (q > 0) col_product<Num, M>(r, a, cp, cl.base);
 #pragma unroll
@@ -327,6 +330,17 @@ __global__ void __launch_bounds__(128, cols_min_ctas<M>(false)) k_reduced_cols(c
     const size_t s = cl.live ? (size_t)cl.sys : 0, rs = (size_t)g.nsys;
     thomas_cols_body<Num, M, true>(g.ra + s, nullptr, g.rc + s, g.rd + s, g.rc + s, rs * 2 * g.nseg, rs, 2 * g.nseg,
                                    true, g.status, cl);
+}
+
+// M^T lambda = g for the adjoint, from the forward blocks as they are stored:
+// At_q = C_{q-1}^T, Bt_q = B_q^T, Ct_q = A_{q+1}^T; lambda in D, the factors in
+// the workspace (raw).
+template <class Num, int M>
+__global__ void __launch_bounds__(128, cols_min_ctas<M>(false)) k_transposed_cols(const SolveArgs g) {
+    const ColLane cl = col_lane<M>(g.nsys);
+    const size_t s = cl.live ? (size_t)cl.sys : 0, rs = (size_t)g.nsys;
+    thomas_cols_body<Num, M, false, true>(g.c + s - rs, g.b + s, g.a + s + rs, g.d + s, g.cw + s, rs * g.nrow, rs,
+                                          g.nrow, true, g.status, cl);
 }
 
 // Local stage of one segment of one system per group (modi_body, column per
@@ -471,6 +485,12 @@ template <class Num, int M>
 cudaError_t launch_thomas_cols(const SolveArgs& g, const LineStrides& ls) {
     const int tpb = cols_threads<M>(g, 1);
     k_thomas_cols<Num, M><<<cols_grid<M>(g.nsys, tpb), tpb, 0, g.stream>>>(g, ls);
+    return cudaGetLastError();
+}
+template <class Num, int M>
+cudaError_t launch_transposed_cols(const SolveArgs& g) {
+    const int tpb = cols_threads<M>(g, 1);
+    k_transposed_cols<Num, M><<<cols_grid<M>(g.nsys, tpb), tpb, 0, g.stream>>>(g);
     return cudaGetLastError();
 }
 template <class Num, int M>

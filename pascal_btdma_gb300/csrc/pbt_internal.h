@@ -94,6 +94,12 @@ template <class Num, int M> cudaError_t launch_update(const SolveArgs& g);
 constexpr int kColsMaxBlock = PBT_MAX_BLOCK;
 template <class Num, int M> cudaError_t launch_thomas_cols(const SolveArgs& g, const LineStrides& ls);
 template <class Num, int M> cudaError_t launch_modi_cols(const SolveArgs& g);
+// M^T x = d for the blocks in a, b, c (x, d in g.d), raw factors in g.cw: one
+// lane a column, and through the CTA's ring (maps.a over C, maps.c over A, with
+// the block's two indices as separate dimensions).
+template <class Num, int M> cudaError_t launch_transposed_cols(const SolveArgs& g);
+template <class Num, int M>
+cudaError_t launch_transposed_ring(const SolveArgs& g, const LineStrides& ls, const ThomasMaps& maps);
 template <class Num, int M> cudaError_t launch_reduced_cols(const SolveArgs& g);
 // Adjoint (pbt_kernels.cuh: k_adjoint, k_transpose_blocks, k_gradients).
 struct AdjointArgs {

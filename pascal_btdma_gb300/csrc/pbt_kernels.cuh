@@ -2498,9 +2498,9 @@ PBT_UNROLL
 PBT_UNROLL
         for (int i = 0; i < M; ++i) {
             const size_t e = idx + (size_t)(i + M * j) * plane;
-            if (adj.da) adj.da[e] = -lam[i] * xm[j];
+            if (adj.da) adj.da[e] = (q > 0) ? -lam[i] * xm[j] : 0.0;
             if (adj.db) adj.db[e] = -lam[i] * x0[j];
-            if (adj.dc) adj.dc[e] = -lam[i] * xp[j];
+            if (adj.dc) adj.dc[e] = (q + 1 < g.nrow) ? -lam[i] * xp[j] : 0.0;
         }
 }
 

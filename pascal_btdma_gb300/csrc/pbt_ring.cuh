@@ -54,6 +54,15 @@ __device__ __forceinline__ void tma_load_4d(unsigned dst, const CUtensorMap* map
         : "memory");
 }
 
+__device__ __forceinline__ void tma_load_5d(unsigned dst, const CUtensorMap* map, int x, int y, int z, int w, int v,
+                                            unsigned bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(dst),
+        "l"(reinterpret_cast<unsigned long long>(map)), "r"(x), "r"(y), "r"(z), "r"(w), "r"(v), "r"(bar)
+        : "memory");
+}
+
 constexpr int kRingSlots = 8;  // at most
 
 __device__ __forceinline__ unsigned global_ns_low() {
@@ -75,8 +84,12 @@ __device__ __forceinline__ void ring_wait(unsigned bar, unsigned parity, volatil
     }
 }
 
-// The producer warp: every item of both sweeps, in order.
-template <int M>
+// The producer warp: every item of both sweeps, in order.  Transposed (the
+// adjoint): A_q, B_q, C_q are C_{q-1}^T, B_q^T, A_{q+1}^T of the blocks as they
+// are stored; their maps split the planes into the block's two indices, so
+// that a column is a box along the second one, and the rows q - 1 and q + 1
+// past either end come as zeros.
+template <int M, bool Transposed>
 __device__ __forceinline__ void ring_produce(const ThomasMaps& maps, const SolveArgs& g, const LineStrides& ls,
                                              int row_first, int warps, int active, int slots, unsigned ring_s,
                                              unsigned full_s, unsigned empty_s, unsigned turn_s,
@@ -88,16 +101,21 @@ __device__ __forceinline__ void ring_produce(const ThomasMaps& maps, const Solve
     int slot = 0, issued = 0;
     unsigned phase = 1;  // parity of empty[slot] to wait for: a fresh barrier passes parity 1
     bool ok = true;
-    auto issue = [&](const CUtensorMap* map, int row, int z) {
+    auto issue = [&](const CUtensorMap* map, int row, int j, bool block) {
         ring_wait(empty_s + 8u * slot, phase, failed);
         ok = __all_sync(0xffffffffu, !*failed);
         if (!ok) return;
         fence_proxy_async_shared();
         if (lane == 0) mbar_expect_tx(full_s + 8u * slot, item_bytes * active);
         __syncwarp();
-        if (lane < active)
-            tma_load_4d(ring_s + slot_bytes * slot + item_bytes * lane, map, x, row_first ? row : outer,
-                        row_first ? outer : row, z, full_s + 8u * slot);
+        if (lane < active) {
+            const unsigned dst = ring_s + slot_bytes * slot + item_bytes * lane;
+            const int y = row_first ? row : outer, z = row_first ? outer : row;
+            if (Transposed && block)
+                tma_load_5d(dst, map, x, y, z, j, 0, full_s + 8u * slot);
+            else
+                tma_load_4d(dst, map, x, y, z, j * M, full_s + 8u * slot);
+        }
         ++issued;
         if (++slot == slots) {
             slot = 0;
@@ -105,18 +123,18 @@ __device__ __forceinline__ void ring_produce(const ThomasMaps& maps, const Solve
         }
     };
     for (int q = 0; q < N && ok; ++q) {
-        issue(&maps.d, q, 0);
-        for (int j = 0; j < M && ok; ++j) issue(&maps.b, q, j * M);
-        for (int j = 0; j < M && ok; ++j) issue(&maps.a, q, j * M);
-        for (int j = 0; j < M && ok; ++j) issue(&maps.c, q, j * M);
+        issue(&maps.d, q, 0, false);
+        for (int j = 0; j < M && ok; ++j) issue(&maps.b, q, j, true);
+        for (int j = 0; j < M && ok; ++j) issue(&maps.a, Transposed ? q - 1 : q, j, true);
+        for (int j = 0; j < M && ok; ++j) issue(&maps.c, Transposed ? q + 1 : q, j, true);
     }
     if (ok) {
         ring_wait(turn_s, 0, failed);
         ok = __all_sync(0xffffffffu, !*failed);
     }
     for (int q = N - 2; q >= 0 && ok; --q) {
-        issue(&maps.d, q, 0);
-        for (int j = 0; j < M && ok; ++j) issue(&maps.w, q, j * M);
+        issue(&maps.d, q, 0, false);
+        for (int j = 0; j < M && ok; ++j) issue(&maps.w, q, j, false);
     }
     // No copy may land after the CTA has ended: wait (bounded) for the last ones.
     if (lane == 0) {
@@ -137,7 +155,7 @@ __host__ __device__ constexpr bool ring_step() {
     return Num::kConv && M >= 4;
 }
 
-template <class Num, int M>
+template <class Num, int M, bool Transposed>
 __global__ void __launch_bounds__(256, 2) k_thomas_ring(const __grid_constant__ ThomasMaps maps, const SolveArgs g,
                                                         const LineStrides ls, int row_first, int slots) {
     using T = typename Num::T;
@@ -160,7 +178,7 @@ __global__ void __launch_bounds__(256, 2) k_thomas_ring(const __grid_constant__ 
     }
     __syncthreads();
     if (w == warps) {
-        ring_produce<M>(maps, g, ls, row_first, warps, active, slots, smem_u32(ring), full_s, empty_s, turn_s,
+        ring_produce<M, Transposed>(maps, g, ls, row_first, warps, active, slots, smem_u32(ring), full_s, empty_s, turn_s,
                         &failed);
         return;
     }
@@ -309,8 +327,9 @@ __global__ void __launch_bounds__(256, 2) k_thomas_ring(const __grid_constant__ 
 // Consumer threads a CTA: as in_step_tpb, at most 224 (with the producer, two
 // CTAs of 256 threads of 128 registers an SM), so that the CTAs make whole
 // waves; as many ring slots as two CTAs an SM leave shared memory for.
-template <class Num, int M>
-cudaError_t launch_thomas_ring(const SolveArgs& g, const LineStrides& ls, const ThomasMaps& maps, int row_first) {
+template <class Num, int M, bool Transposed>
+cudaError_t launch_ring(const SolveArgs& g, const LineStrides& ls, const ThomasMaps& maps, int row_first) {
+    const auto kernel = k_thomas_ring<Num, M, Transposed>;
     const long long sms = g.sms > 0 ? g.sms : 1, cap = 224;
     const long long waves = (g.nsys + cap * sms - 1) / (cap * sms);
     const int warps = (int)((((long long)g.nsys + waves * sms - 1) / (waves * sms) + 31) / 32);
@@ -320,11 +339,19 @@ cudaError_t launch_thomas_ring(const SolveArgs& g, const LineStrides& ls, const 
     size_t slots = (budget - fixed) / slot;
     if (slots > kRingSlots) slots = kRingSlots;
     const size_t smem = fixed + slots * slot;
-    cudaError_t e = cudaFuncSetAttribute(k_thomas_ring<Num, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     const unsigned grid = (unsigned)(((g.nsys + 31) / 32 + warps - 1) / warps);
-    k_thomas_ring<Num, M><<<grid, 32 * (warps + 1), smem, g.stream>>>(maps, g, ls, row_first, (int)slots);
+    kernel<<<grid, 32 * (warps + 1), smem, g.stream>>>(maps, g, ls, row_first, (int)slots);
     return cudaGetLastError();
+}
+template <class Num, int M>
+cudaError_t launch_thomas_ring(const SolveArgs& g, const LineStrides& ls, const ThomasMaps& maps, int row_first) {
+    return launch_ring<Num, M, false>(g, ls, maps, row_first);
+}
+template <class Num, int M>
+cudaError_t launch_transposed_ring(const SolveArgs& g, const LineStrides& ls, const ThomasMaps& maps) {
+    return launch_ring<Num, M, true>(g, ls, maps, 1);
 }
 
 }  // namespace pbt
