@@ -157,10 +157,11 @@ void pbt_plan_desc_init(pbt_plan_desc* desc);
  * the GPU with one thread per system (nsys >= 128 * SMs, 19456 on a GB300)
  * is solved one segment per line whatever nseg says: the single-segment
  * method does ~40 % of the two-stage method's arithmetic and gives the same x
- * to rounding.  Non-cyclic FP64 and PBT_PREC_FF plans that are not in place do
- * so from m = 3 and fewer systems on, where that is faster (8 to 78 * SMs by m and
- * precision).  PBT_FLAG_REFERENCE_METHOD keeps the nseg segments (and the
- * reference's in-place A', C' with PBT_FLAG_INPLACE). */
+ * to rounding.  Smaller non-cyclic FP64 and PBT_PREC_FF batches that are not in
+ * place are solved in one segment, or by elimination from both ends of the line
+ * at once, where that is faster (same x to rounding).
+ * PBT_FLAG_REFERENCE_METHOD keeps the nseg segments (and the reference's
+ * in-place A', C' with PBT_FLAG_INPLACE). */
 int pbt_plan_create(pbt_plan** plan, int m, int nsys, int nrow, int nseg);
 
 /* As pbt_plan_create with every option of pbt_plan_desc. */
@@ -183,7 +184,10 @@ int pbt_solve_noncyclic(pbt_plan* plan, double* a, double* b, double* c, double*
 
 /* Replaces solve_noncyclic_profiled (pascal_btdma_cuda.cu:1047-1061) and
  * btdma_many_mpi_gpu_v2_profiled (mod_btdma_gpu_v2.f90:169-198).  `timings`
- * may be NULL.  Synchronises `stream`. */
+ * may be NULL.  Synchronises `stream`.  On a batch below 128 * SMs systems the
+ * nseg > 1 segments are solved as such, for their phases, also where
+ * pbt_solve_noncyclic would not keep them (the first such call allocates
+ * their workspace). */
 int pbt_solve_noncyclic_profiled(pbt_plan* plan, double* a, double* b, double* c, double* d,
                                  int m, int nsys, int nrow, pbt_timings* timings, void* stream);
 

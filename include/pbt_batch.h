@@ -16,11 +16,13 @@
  * that decouple from it (B = I, A = C = 0, d = 0); unpack returns only the
  * system's own rows.
  *
- * The solve runs, per block size present (largest total cost first), a
- * persistent launch over the local-stage items (the warp that completes a
- * tile's last segment also solves the tile's reduced system) and a
- * launch over the update items, on the caller's stream; each
- * launch carries one block size's code.
+ * Where the batch is large enough for its longest line, the block sizes up to 6
+ * are solved in one launch with one lane per block column, lines of several
+ * segments by elimination from both ends instead.  Otherwise, and for the
+ * larger block sizes, the solve runs, per block size present (largest total
+ * cost first), a persistent launch over the local-stage items (the warp that
+ * completes a tile's last segment also solves the tile's reduced system) and a
+ * launch over the update items; all on the caller's stream.
  *
  * Tuning (pbt_batch_tuning): the number of segments of each tile is
  * round(N_max / seg_len[m]) (one segment when seg_len[m] <= 0), so long lines
@@ -76,7 +78,7 @@ int pbt_batch_pack(pbt_batch* batch, const double* ua, const double* ub, const d
 int pbt_batch_unpack(pbt_batch* batch, const double* pd, double* ud, void* stream);
 
 /* Solve every system of the batch in place on packed arrays: one memset of
- * the queue state and up to two launches per block size present, no host
+ * the queue state and one launch, or up to two per block size present, no host
  * synchronisation. */
 int pbt_batch_solve(pbt_batch* batch, const double* pa, const double* pb, const double* pc, double* pd,
                     void* stream);
@@ -89,8 +91,9 @@ int pbt_batch_solve(pbt_batch* batch, const double* pa, const double* pb, const 
  * that order. */
 int pbt_batch_status(pbt_batch* batch, long long* nsingular, int* timed_out);
 
-/* Shape of the schedule: tiles, stage-1 and stage-3 items, CTAs of the
- * largest persistent launch of the last solve (0 before the first). */
+/* Shape of the schedule: tiles, stage-1 items (of the single launch, too) and
+ * stage-3 items, CTAs of the largest launch of the last solve (0 before the
+ * first). */
 int pbt_batch_info(const pbt_batch* batch, int* ntiles, int* n_items1, int* n_items3, int* grid_ctas);
 
 #ifdef __cplusplus

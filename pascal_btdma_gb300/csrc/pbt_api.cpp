@@ -47,6 +47,7 @@ struct pbt_plan {
     int device = 0;
     int sms = 0;          // multiprocessors of `device`
     bool thomas = false;  // single-segment plain block Thomas path
+    bool twisted = false;  // thomas, eliminated from both ends (nseg > 1 only)
     bool lines = false;   // strided lines and the fused adjoint: nseg = 1, or a batch that fills the GPU
     bool cyclic_thomas = false;  // single-segment periodic block Thomas (k_thomas_cyclic)
     double* aw = nullptr;  // factor workspace (nullptr when in place)
@@ -326,11 +327,17 @@ cudaError_t run_thomas_cols(int arith, int m, const pbt::SolveArgs& g, const pbt
     }
     PBT_DISPATCH_PLAIN_M2(pbt::F64, launch_thomas_cols, g, ls)
 }
-cudaError_t run_transposed_cols(int arith, int m, const pbt::SolveArgs& g) {
+cudaError_t run_twist_cols(int arith, int m, const pbt::SolveArgs& g) {
     if (arith == kFF) {
-        PBT_DISPATCH_PLAIN_M2(pbt::FF, launch_transposed_cols, g)
+        PBT_DISPATCH_PLAIN_M2(pbt::FF, launch_twist_cols, g)
     }
-    PBT_DISPATCH_PLAIN_M2(pbt::F64, launch_transposed_cols, g)
+    PBT_DISPATCH_PLAIN_M2(pbt::F64, launch_twist_cols, g)
+}
+cudaError_t run_transposed_cols(int arith, int m, const pbt::SolveArgs& g, int twisted) {
+    if (arith == kFF) {
+        PBT_DISPATCH_PLAIN_M2(pbt::FF, launch_transposed_cols, g, twisted)
+    }
+    PBT_DISPATCH_PLAIN_M2(pbt::F64, launch_transposed_cols, g, twisted)
 }
 cudaError_t run_modi_cols(int arith, int m, const pbt::SolveArgs& g) {
     if (arith == kFF) {
@@ -458,8 +465,8 @@ bool encode_block_rows(CUtensorMap* tm, const double* base, int nsys, int nrow, 
 // blocks: by column lanes or through the ring where the forward solve takes
 // them; false: neither, not launched.
 bool transposed_launch(const pbt_plan* p, int arith, int m, const pbt::SolveArgs& g, cudaError_t* e) {
-    if (thomas_cols(p, arith, m)) {
-        *e = run_transposed_cols(arith, m, g);
+    if (p->twisted || thomas_cols(p, arith, m)) {
+        *e = run_transposed_cols(arith, m, g, p->twisted);
         return true;
     }
     if (!g.tpb_auto || (p->desc.flags & (PBT_FLAG_DIRECT_LOADS | PBT_FLAG_STAGED_LOADS)) ||
@@ -488,6 +495,7 @@ bool transposed_launch(const pbt_plan* p, int arith, int m, const pbt::SolveArgs
 
 cudaError_t thomas_launch(const pbt_plan* p, int arith, int m, const pbt::SolveArgs& g) {
     const pbt::LineStrides plain{g.nsys, 1, 0, g.nsys, (long long)g.nsys * g.nrow};
+    if (p->twisted) return run_twist_cols(arith, m, g);
     if (thomas_cols(p, arith, m)) return run_thomas_cols(arith, m, g, plain);
     cudaError_t e;
     if (ring_launch(p, arith, m, g, plain, &e)) return e;
@@ -563,15 +571,41 @@ bool fills_gpu(int nsys, int sms) {
 //     -> 30475 (8).
 // m <= 2 keeps its segments up to fills_gpu's line (FP64 m = 2, 14000 x 512 in
 // 16 1222 -> 1686; float-float 13000 626 -> 628).
-// Not for plans whose factors the caller gets (in place) or that ask for the
-// reference method.
 bool one_segment_pays(const pbt_plan_desc& d, int sms) {
-    if (d.precision == PBT_PREC_FP32_REFINE ||
-        (d.flags & (PBT_FLAG_CYCLIC | PBT_FLAG_INPLACE | PBT_FLAG_REFERENCE_METHOD)))
-        return false;
     static const int ff[] = {128, 128, 30, 30, 14, 8, 11, 9}, fp64[] = {128, 128, 22, 78, 18, 13, 11, 8};
     const int line = (d.precision == PBT_PREC_FF ? ff : fp64)[d.m < 8 ? d.m - 1 : 7];
     return d.nsys >= line * (long long)(sms > 0 ? sms : 152);
+}
+
+// Plans whose method is the library's choice: nseg > 1, non-cyclic, FP64 or
+// float-float, the factors not the caller's (in place), the reference method
+// not asked for.
+bool method_free(const pbt_plan_desc& d) {
+    return d.nseg > 1 && d.precision != PBT_PREC_FP32_REFINE &&
+           !(d.flags & (PBT_FLAG_CYCLIC | PBT_FLAG_INPLACE | PBT_FLAG_REFERENCE_METHOD));
+}
+// Whether such a plan solves its lines from both ends at once (the twisted form
+// of pbt_cols.cuh: half the chain of one segment at the same arithmetic, against
+// the two-stage method's 2.4 times): while its pairs of warps are resident
+// together (three rounds of them for m <= 3, whose rows are short), if one
+// segment pays at all or the chain of half the rows ends before the two-stage
+// method's chain and work (ColsCost).  us, segments / one segment -> twisted:
+// float-float m = 3, 6500 x 512 in 16 1121 / 1013 -> 632, 1500 261 / 850 -> 425
+// (stays in segments); m = 5, 1500 x 256 in 3 627 / 568 -> 329, 8000 x 512 in 16
+// 3507 / 2527 -> 2537 (stays in one); FP64 m = 4, 4000 x 512 in 16 2333 / 2233
+// -> 1961, 8000 4403 / 4549 -> 5872 (past residency); m = 8, 800 x 512 in 16
+// 5035 / 6325 -> 3501.
+bool twisted_pays(const pbt_plan_desc& d, int sms) {
+    if (!method_free(d) || (d.flags & (PBT_FLAG_DIRECT_LOADS | PBT_FLAG_STAGED_LOADS)) || d.threads_per_block) return false;
+    const int arith = arith_of(d.precision), per = 32 / (d.m + 1);
+    const long long n = sms > 0 ? sms : 152, warps = 2LL * ((d.nsys + per - 1) / per);
+    if (!cols_pay(arith, d.m, d.nsys, false, sms) || warps > n * (d.m <= 3 ? 48 : d.m <= 6 ? 16 : 12)) return false;
+    if (one_segment_pays(d, sms)) return true;
+    const pbt::ColsCost& c = arith == kFF ? pbt::kColsFF : pbt::kColsF64;
+    const double rows = 1e-3 * d.nsys * d.nrow, chain = c.chain[d.m - 1];
+    const double both_ends = std::fmax(0.5 * d.nrow * chain, rows * c.row[d.m - 1]);
+    const double segments = std::fmax((1.8 * d.nrow / d.nseg + 2.0 * d.nseg + 12.0) * chain, rows * c.segmented[d.m - 1]);
+    return both_ends < segments;
 }
 
 // The local-stage and update launches put the segments in gridDim.y.
@@ -876,6 +910,23 @@ int solve_core(pbt_plan* p, double* a, double* b, double* c, double* d, int m, i
     if (timed && !evs.ok) return fail(PBT_ECUDA, "solve_profiled: cudaEventCreate failed");
     auto mark = [&](int i) -> cudaError_t { return timed ? cudaEventRecord(evs.ev[i], s) : cudaSuccess; };
 
+    // A profiled solve reports the phases of the segments that the caller asked
+    // for: where the library's own measurements would solve a batch that does
+    // not fill the GPU without them, it runs the two-stage method (whose
+    // workspace the first such call allocates).
+    const bool phases = timed && p->thomas && !p->lines;
+    if (phases && !p->ra) {
+        const size_t mm = (size_t)m * m, rows = (size_t)nsys * nrow, rrows = (size_t)nsys * 2 * ds.nseg, had = p->bytes;
+        if ((rc = alloc(p, &p->aw, mm * rows)) || (rc = alloc(p, &p->rc, mm * rrows)) ||
+            (rc = alloc(p, &p->rd, (size_t)m * rrows)) || (rc = alloc(p, &p->ra, mm * rrows))) {
+            cudaFree(p->aw);
+            cudaFree(p->rc);
+            cudaFree(p->rd);
+            p->aw = p->rc = p->rd = nullptr;
+            p->bytes = had;
+            return rc;
+        }
+    }
     cudaError_t e;
     if ((e = mark(0)) != cudaSuccess) return cuda_fail(e, "cudaEventRecord");
     if (ds.precision == PBT_PREC_FP32_REFINE) {
@@ -883,7 +934,7 @@ int solve_core(pbt_plan* p, double* a, double* b, double* c, double* d, int m, i
         if (rc) return rc;
         for (int i = 1; i < 5; ++i)
             if ((e = mark(i)) != cudaSuccess) return cuda_fail(e, "cudaEventRecord");
-    } else if (p->thomas || p->cyclic_thomas) {
+    } else if ((p->thomas && !phases) || p->cyclic_thomas) {
         const pbt::SolveArgs g = make_args(p, a, b, c, d, s, nsys);
         e = p->thomas ? thomas_launch(p, arith_of(ds.precision), m, g)
                       : run_thomas_cyclic(arith_of(ds.precision), m, g);
@@ -932,7 +983,7 @@ int solve_core(pbt_plan* p, double* a, double* b, double* c, double* d, int m, i
         for (int i = 0; i < 4; ++i) cudaEventElapsedTime(&ms[i], evs.ev[i], evs.ev[i + 1]);
         float tot = 0;
         cudaEventElapsedTime(&tot, evs.ev[0], evs.ev[4]);
-        if (p->thomas || p->cyclic_thomas) {
+        if ((p->thomas && !phases) || p->cyclic_thomas) {
             // One fused launch: all of it is local compute.
             t->local_compute = tot * 1e-3;
             t->forward_exchange = t->reduced_compute = t->backward_exchange = t->update_compute = 0.0;
@@ -981,12 +1032,13 @@ int pbt_plan_create_ex(pbt_plan** out, const pbt_plan_desc* desc) {
     const bool cyclic = (d.flags & PBT_FLAG_CYCLIC) != 0;
     // nseg is the reference's decomposition of a line over MPI ranks.  On one
     // GPU, a batch with enough systems (fills_gpu, one_segment_pays) is solved
-    // one segment per line (the method of nseg = 1: ~40 % of the two-stage
-    // method's arithmetic, same x to rounding) unless
+    // one segment per line (the method of nseg = 1, or from both ends: ~40 % of the
+    // two-stage method's arithmetic, same x to rounding) unless
     // PBT_FLAG_REFERENCE_METHOD asks for the segments.
     const bool full = d.nseg == 1 || (!(d.flags & PBT_FLAG_REFERENCE_METHOD) && fills_gpu(d.nsys, p->sms) &&
                                       (!cyclic || d.nrow >= 3));
-    const bool one_seg = full || one_segment_pays(d, p->sms);
+    p->twisted = !full && twisted_pays(d, p->sms);
+    const bool one_seg = full || p->twisted || (method_free(d) && one_segment_pays(d, p->sms));
     p->thomas = one_seg && !cyclic && !(d.flags & PBT_FLAG_REFERENCE_METHOD);
     p->lines = p->thomas && full;
     p->cyclic_thomas = one_seg && cyclic;

@@ -22,6 +22,7 @@ struct pbt_batch {
     int off3[PBT_MAX_BLOCK + 1] = {}, cnt3[PBT_MAX_BLOCK + 1] = {};
     int rows3[PBT_MAX_BLOCK + 1] = {};  // rows of the longest segment of items3
     std::vector<int> order;
+    int off_cols = 0, cnt_cols = 0;  // items1 of k_batch_cols (0: not used)
     std::vector<long long> user_mat_off, user_vec_off;
     long long user_mat = 0, user_vec = 0, packed_mat = 0, packed_vec = 0, red_mat = 0, red_vec = 0;
     // device
@@ -116,6 +117,22 @@ void free_batch(pbt_batch* b) {
     cudaFree(b->rd);
 }
 
+// Whether the tiles of block sizes up to kBatchColsMaxBlock are solved by
+// k_batch_cols: when the longest chain (half the rows of a tile of several
+// segments, eliminated from both ends) ends within the time that the segmented
+// launches would take for all of them.
+bool cols_solve(const std::vector<pbt::BatchTile>& tiles, int precision) {
+    const pbt::ColsCost& c = precision == PBT_PREC_FF ? pbt::kColsFF : pbt::kColsF64;
+    double chain = 0.0, cols = 0.0, segmented = 0.0;  // us
+    for (const auto& t : tiles) {
+        if (t.m > pbt::kBatchColsMaxBlock) continue;
+        chain = std::max(chain, c.chain[t.m - 1] * t.rows / (t.nseg > 1 ? 2 : 1));
+        cols += 32e-3 * c.row[t.m - 1] * t.rows;
+        segmented += 32e-3 * c.segmented[t.m - 1] * t.rows;
+    }
+    return std::max(chain, cols) < segmented;
+}
+
 int check(const pbt_batch* b) {
     if (!b || b->magic != kBatchMagic) return bfail(PBT_ESTATE, "batch: null, destroyed or corrupt handle");
     return PBT_OK;
@@ -198,14 +215,8 @@ int pbt_batch_create(pbt_batch** out, int nsys, const int* m, const int* nrow, i
         t.nseg = P;
         t.mat_off = mat_off;
         t.vec_off = vec_off;
-        t.red_mat_off = red_m;
-        t.red_vec_off = red_v;
         mat_off += 32LL * t.rows * mm * mm;
         vec_off += 32LL * t.rows * mm;
-        if (P > 1) {
-            red_m += 32LL * 2 * P * mm * mm;
-            red_v += 32LL * 2 * P * mm;
-        }
         chunk_start.push_back((int)chunks);
         chunks += (t.rows + pbt::kPackRows - 1) / pbt::kPackRows;
         for (int l = 0; l < 32; ++l) {
@@ -216,6 +227,16 @@ int pbt_batch_create(pbt_batch** out, int nsys, const int* m, const int* nrow, i
         k += lanes;
     }
     b->ntiles = (int)tiles.size();
+    const bool cols = cols_solve(tiles, precision);
+    const auto by_cols = [&](const pbt::BatchTile& t) { return cols && t.m <= pbt::kBatchColsMaxBlock; };
+    for (auto& t : tiles) {
+        t.red_mat_off = red_m;
+        t.red_vec_off = red_v;
+        if (t.nseg > 1 && !by_cols(t)) {
+            red_m += 32LL * 2 * t.nseg * t.m * t.m;
+            red_v += 32LL * 2 * t.nseg * t.m;
+        }
+    }
     b->packed_mat = mat_off;
     b->packed_vec = vec_off;
     b->red_mat = red_m;
@@ -237,7 +258,7 @@ int pbt_batch_create(pbt_batch** out, int nsys, const int* m, const int* nrow, i
         double total = 0.0;
         for (int t = 0; t < b->ntiles; ++t) {
             const auto& tl = tiles[t];
-            if (tl.m != mm) continue;
+            if (tl.m != mm || by_cols(tl)) continue;
             const double w = (double)tl.m * tl.m * tl.m;
             if (tl.nseg == 1) {
                 it1.push_back({t, -1, w * tl.rows});
@@ -262,6 +283,22 @@ int pbt_batch_create(pbt_batch** out, int nsys, const int* m, const int* nrow, i
         b->cnt1[mm] = (int)items1.size() - b->off1[mm];
         b->cnt3[mm] = (int)items3.size() - b->off3[mm];
         by_cost.push_back({total, mm});
+    }
+    if (cols) {
+        // Longest chain first: the order in which the CTAs start.
+        const pbt::ColsCost& c = precision == PBT_PREC_FF ? pbt::kColsFF : pbt::kColsF64;
+        std::vector<It> it1;
+        for (int t = 0; t < b->ntiles; ++t) {
+            const auto& tl = tiles[t];
+            if (!by_cols(tl)) continue;
+            const int per = (32 / (tl.m + 1)) * (tl.nseg > 1 ? 1 : 2);  // systems an item
+            for (int k = 0; k * per < tl.lanes; ++k)
+                it1.push_back({t, k, c.chain[tl.m - 1] * tl.rows / (tl.nseg > 1 ? 2 : 1)});
+        }
+        std::stable_sort(it1.begin(), it1.end(), [](const It& x, const It& y) { return x.cost > y.cost; });
+        b->off_cols = (int)items1.size();
+        b->cnt_cols = (int)it1.size();
+        for (const auto& i : it1) items1.push_back(make_int2(i.t, i.s));
     }
     std::stable_sort(by_cost.begin(), by_cost.end(), [](const std::pair<double, int>& x, const std::pair<double, int>& y) {
         return x.first > y.first;
@@ -380,6 +417,16 @@ int pbt_batch_solve(pbt_batch* b, const double* pa, const double* pb, const doub
     ba.status = b->status;
     ba.seg_done = b->state + 2 + kHeads;
     b->last_grid = 0;
+    if (b->cnt_cols > 0) {
+        ba.items1 = b->items1 + b->off_cols;
+        ba.items3 = nullptr;
+        ba.n1 = b->cnt_cols;
+        ba.n3 = ba.rows3 = 0;
+        ba.head1 = nullptr;
+        if ((e = pbt::launch_batch_cols(ba, b->precision == PBT_PREC_FF, s)) != cudaSuccess)
+            return bcuda(e, "batch_solve: launch");
+        b->last_grid = b->cnt_cols;
+    }
     for (int mm : b->order) {
         ba.items1 = b->items1 + b->off1[mm];
         ba.items3 = b->items3 + b->off3[mm];

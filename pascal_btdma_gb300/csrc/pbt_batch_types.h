@@ -51,6 +51,11 @@ struct PackArgs {
 };
 constexpr int kPackRows = 64;
 
+// Block sizes up to this may be solved by k_batch_cols (pbt_batch_cols.cu):
+// one CTA of two warps per item (tile, group of systems) in items1.
+constexpr int kBatchColsMaxBlock = 6;
+cudaError_t launch_batch_cols(const BatchArgs& ba, int ff, cudaStream_t s);
+
 // The launches of block size M (pbt_batch.cuh; instantiated with the other
 // kernels of (Num, M) in pbt_inst.cu).
 template <class Num, int M>

@@ -46,10 +46,9 @@ struct ColLane {
     bool live;
 };
 template <int M>
-__device__ __forceinline__ ColLane col_lane(long long nsys) {
+__device__ __forceinline__ ColLane col_lane(long long nsys, long long warp) {
     constexpr int G = M + 1, S = cols_systems<M>();
     const int lane = threadIdx.x & 31;
-    const long long warp = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     ColLane c;
     const bool idle = lane >= S * G;
     const int g = idle ? S - 1 : lane / G;
@@ -58,6 +57,10 @@ __device__ __forceinline__ ColLane col_lane(long long nsys) {
     c.sys = warp * S + g;
     c.live = !idle && c.sys < nsys;
     return c;
+}
+// This warp's number in the grid.
+__device__ __forceinline__ long long grid_warp() {
+    return (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
 }
 
 // M values `stride` apart at p (zeros on a lane that is not live), raw.
@@ -169,18 +172,24 @@ __device__ __forceinline__ void col_product2(typename Num::Acc (&acc)[M], typena
         }
 }
 
-// A lane's outcome of its group, reported once a system: the group's pivots
-// and the range check of the values it wrote.
-template <class Num, int M>
-__device__ __forceinline__ void col_report(unsigned long long* status, unsigned bad, unsigned amax, bool whole,
-                                           const ColLane& cl) {
+// The outcome of a lane's group: its pivots and the largest value it wrote.
+template <int M>
+__device__ __forceinline__ void col_merge(unsigned& bad, unsigned& amax, const ColLane& cl) {
     unsigned b = 0, a = 0;
 #pragma unroll
     for (int k = 0; k <= M; ++k) {
         b |= __shfl_sync(0xffffffffu, bad, cl.base + k);
         a = max(a, __shfl_sync(0xffffffffu, amax, cl.base + k));
     }
-    if (cl.live && cl.j == 0) report_status(status, b | range_bits<Num>(a, whole));
+    bad = b;
+    amax = a;
+}
+// Reported once a system, with the range check of the values it wrote.
+template <class Num, int M>
+__device__ __forceinline__ void col_report(unsigned long long* status, unsigned bad, unsigned amax, bool whole,
+                                           const ColLane& cl) {
+    col_merge<M>(bad, amax, cl);
+    if (cl.live && cl.j == 0) report_status(status, bad | range_bits<Num>(amax, whole));
 }
 
 // Rows of C' and y that the backward sweep has in flight.
@@ -193,10 +202,19 @@ __host__ __device__ constexpr int cols_ahead() {
 // system's first row; Reduced: the reduced system of the two-stage method (B =
 // I, everything raw; A, C', d in RA, RC, RD); Transposed: A, B and C hold the
 // transposed blocks (column j of a block is row j of what is stored).
-template <class Num, int M, bool Reduced, bool Transposed = false>
+//
+// Twisted: the line is eliminated from both ends at once, by two warps of a
+// CTA (the pair's `side` 0 from the first row on, 1 from the last row on with A
+// and C in each other's place and a negative row stride), N rows each.  Where
+// they meet, x = y - P x' on either side (P the last C', x', P' and y' the
+// other side's), so x = (I - P P')^{-1} (y - P y'); then both substitute back
+// outwards.  Half the chain of block Thomas at the same arithmetic.  `sh`: the
+// pair's exchange, 2 x 32 lanes x M values.
+template <class Num, int M, bool Reduced, bool Transposed = false, bool Twisted = false>
 __device__ __forceinline__ void thomas_cols_body(const double* A, const double* B, const double* C, double* D,
-                                                 double* CW, size_t plane, size_t rs, int N, bool raw,
-                                                 unsigned long long* status, const ColLane& cl) {
+                                                 double* CW, size_t plane, ptrdiff_t rs, int N, bool raw,
+                                                 unsigned long long* status, const ColLane& cl, int side = 0,
+                                                 double* sh = nullptr) {
     using T = typename Num::T;
     using Acc = typename Num::Acc;
     const bool rhs = cl.j == M;
@@ -216,9 +234,9 @@ __device__ __forceinline__ void thomas_cols_body(const double* A, const double* 
         col_load<M>(vb, pb, plane, cl.live && rhs);
     else
         col_load<M>(vb, pb, eb, cl.live);
-    col_load<M>(vc, pc, es, mat && N > 1);
+    col_load<M>(vc, pc, es, mat && (Twisted || N > 1));
     for (int q = 0; q < N; ++q) {
-        const size_t o = (size_t)q * rs;
+        const ptrdiff_t o = q * rs;
         const bool last = q == N - 1;
         T a[M];
         Acc r[M], x[1][M];
@@ -233,13 +251,13 @@ __device__ __forceinline__ void thomas_cols_body(const double* A, const double* 
         }
         // The next row's inputs, on their way while this row is eliminated.
         if (!last) {
-            const size_t p = o + rs;
+            const ptrdiff_t p = o + rs;
             col_load<M>(va, pa + p, es, mat);
             if constexpr (Reduced)
                 col_load<M>(vb, pb + p, plane, cl.live && rhs);
             else
                 col_load<M>(vb, pb + p, eb, cl.live);
-            col_load<M>(vc, pc + p, es, mat && q + 2 < N);
+            col_load<M>(vc, pc + p, es, mat && (Twisted || q + 2 < N));
         }
         if (q > 0) col_product<Num, M>(r, a, cp, cl.base);
 #pragma unroll
@@ -247,7 +265,7 @@ __device__ __forceinline__ void thomas_cols_body(const double* A, const double* 
         col_gesv<Num, M, 1>(r, x, cl, bad);
 #pragma unroll
         for (int i = 0; i < M; ++i) cp[i] = Num::fin(x[0][i]);
-        if (cl.live && (rhs || !last)) {
+        if (cl.live && (Twisted ? !last : rhs || !last)) {
 #pragma unroll
             for (int i = 0; i < M; ++i) {
                 double* const p = pw + o + (size_t)i * plane;
@@ -256,6 +274,34 @@ __device__ __forceinline__ void thomas_cols_body(const double* A, const double* 
                     Num::sts(p, cp[i]);
                 else
                     Num::out(p, cp[i]);
+            }
+        }
+    }
+    if constexpr (Twisted) {
+        // This side's P and y (cp) against the other's, lane by lane.
+        double* const mine = sh + (side * 32 + (threadIdx.x & 31)) * M;
+        const double* const other = sh + ((side ^ 1) * 32 + (threadIdx.x & 31)) * M;
+#pragma unroll
+        for (int i = 0; i < M; ++i) Num::sts(mine + i, cp[i]);
+        __syncthreads();
+        T oc[M];
+        Acc r[M], x[1][M];
+#pragma unroll
+        for (int i = 0; i < M; ++i) {
+            oc[i] = Num::lds(other + i);
+            r[i] = rhs ? Num::acc(cp[i]) : Num::acc(i == cl.j ? Num::one() : Num::zero());
+        }
+        col_product<Num, M>(r, cp, oc, cl.base);
+#pragma unroll
+        for (int i = 0; i < M; ++i) x[0][i] = Num::asel(rhs, r[i], Num::acc0());
+        col_gesv<Num, M, 1>(r, x, cl, bad);
+        const ptrdiff_t o = (N - 1) * rs;
+#pragma unroll
+        for (int i = 0; i < M; ++i) {
+            cp[i] = Num::fin(x[0][i]);
+            if (cl.live && rhs) {
+                amax = max(amax, Num::mag(cp[i]));
+                Num::out(pw + o + (size_t)i * plane, cp[i]);
             }
         }
     }
@@ -271,7 +317,7 @@ __device__ __forceinline__ void thomas_cols_body(const double* A, const double* 
     double bc[kAhead][M], by[kAhead];
     auto fetch = [&](int slot, int q) {
         const bool on = mat && q >= 0;
-        const size_t o = (size_t)(q >= 0 ? q : 0) * rs;
+        const ptrdiff_t o = (q >= 0 ? q : 0) * rs;
         by[slot] = on ? py[o] : 0.0;
 #pragma unroll
         for (int k = 0; k < M; ++k) bc[slot][k] = on ? pr[o + (size_t)(M * k) * plane] : 0.0;
@@ -285,7 +331,7 @@ __device__ __forceinline__ void thomas_cols_body(const double* A, const double* 
         for (int s = 0; s < kAhead; ++s) {
             const int q = q0 - s;
             if (q >= 0) {
-                const size_t o = (size_t)q * rs;
+                const ptrdiff_t o = q * rs;
                 Acc t = Num::acc(Num::from_raw(by[s]));
 #pragma unroll
                 for (int k = 0; k < M; ++k) {
@@ -307,7 +353,21 @@ __device__ __forceinline__ void thomas_cols_body(const double* A, const double* 
             }
         }
     }
-    col_report<Num, M>(status, bad, amax, true, cl);
+    if constexpr (Twisted) {
+        // The line's outcome, both sides together, reported by side 0.
+        col_merge<M>(bad, amax, cl);
+        unsigned* const u = reinterpret_cast<unsigned*>(sh) + 2 * (threadIdx.x & 31);
+        __syncthreads();  // the exchange has been read
+        if (side == 1) {
+            u[0] = bad;
+            u[1] = amax;
+        }
+        __syncthreads();
+        if (side == 0 && cl.live && cl.j == 0)
+            report_status(status, bad | u[0] | range_bits<Num>(max(amax, u[1]), true));
+    } else {
+        col_report<Num, M>(status, bad, amax, true, cl);
+    }
 }
 
 // CTAs of four warps an SM holds (the register cap).
@@ -317,7 +377,7 @@ __host__ __device__ constexpr int cols_min_ctas(bool local_stage) {
 }
 template <class Num, int M>
 __global__ void __launch_bounds__(128, cols_min_ctas<M>(false)) k_thomas_cols(const SolveArgs g, const LineStrides ls) {
-    const ColLane cl = col_lane<M>(g.nsys);
+    const ColLane cl = col_lane<M>(g.nsys, grid_warp());
     const long long s = cl.live ? cl.sys : 0;
     const size_t o = (size_t)(s % ls.lin) * (size_t)ls.in + (size_t)(s / ls.lin) * (size_t)ls.out;
     thomas_cols_body<Num, M, false>(g.a + o, g.b + o, g.c + o, g.d + o, g.cw + o, (size_t)ls.elem, (size_t)ls.row,
@@ -326,7 +386,7 @@ __global__ void __launch_bounds__(128, cols_min_ctas<M>(false)) k_thomas_cols(co
 
 template <class Num, int M>
 __global__ void __launch_bounds__(128, cols_min_ctas<M>(false)) k_reduced_cols(const SolveArgs g) {
-    const ColLane cl = col_lane<M>(g.nsys);
+    const ColLane cl = col_lane<M>(g.nsys, grid_warp());
     const size_t s = cl.live ? (size_t)cl.sys : 0, rs = (size_t)g.nsys;
     thomas_cols_body<Num, M, true>(g.ra + s, nullptr, g.rc + s, g.rd + s, g.rc + s, rs * 2 * g.nseg, rs, 2 * g.nseg,
                                    true, g.status, cl);
@@ -337,10 +397,25 @@ __global__ void __launch_bounds__(128, cols_min_ctas<M>(false)) k_reduced_cols(c
 // the workspace (raw).
 template <class Num, int M>
 __global__ void __launch_bounds__(128, cols_min_ctas<M>(false)) k_transposed_cols(const SolveArgs g) {
-    const ColLane cl = col_lane<M>(g.nsys);
+    const ColLane cl = col_lane<M>(g.nsys, grid_warp());
     const size_t s = cl.live ? (size_t)cl.sys : 0, rs = (size_t)g.nsys;
     thomas_cols_body<Num, M, false, true>(g.c + s - rs, g.b + s, g.a + s + rs, g.d + s, g.cw + s, rs * g.nrow, rs,
                                           g.nrow, true, g.status, cl);
+}
+
+// The twisted solve, one pair of warps a CTA; Transposed: of M^T, as above.
+template <class Num, int M, bool Transposed>
+__global__ void __launch_bounds__(64, 2 * cols_min_ctas<M>(false)) k_twist_cols(const SolveArgs g) {
+    __shared__ double sh[2 * 32 * M];
+    const ColLane cl = col_lane<M>(g.nsys, blockIdx.x);
+    const int side = threadIdx.x >> 5, n0 = g.nrow / 2, n = side ? g.nrow - n0 : n0;
+    const ptrdiff_t rs = g.nsys;
+    const size_t plane = (size_t)g.nsys * g.nrow;
+    const ptrdiff_t o = (cl.live ? (ptrdiff_t)cl.sys : 0) + (side ? rs * (g.nrow - 1) : 0);
+    const double* const a = Transposed ? g.c - rs : g.a;  // row q of the lower blocks at a + o + q * rs
+    const double* const c = Transposed ? g.a + rs : g.c;
+    thomas_cols_body<Num, M, false, Transposed, true>((side ? c : a) + o, g.b + o, (side ? a : c) + o, g.d + o,
+                                                      g.cw + o, plane, side ? -rs : rs, n, true, g.status, cl, side, sh);
 }
 
 // Local stage of one segment of one system per group (modi_body, column per
@@ -350,7 +425,7 @@ template <class Num, int M>
 __global__ void __launch_bounds__(128, cols_min_ctas<M>(true)) k_modi_cols(const SolveArgs g) {
     using T = typename Num::T;
     using Acc = typename Num::Acc;
-    const ColLane cl = col_lane<M>(g.nsys);
+    const ColLane cl = col_lane<M>(g.nsys, grid_warp());
     const bool rhs = cl.j == M, mat = cl.live && !rhs, raw = g.factors_raw != 0;
     const int seg = blockIdx.y;
     int f, l;
@@ -488,7 +563,16 @@ cudaError_t launch_thomas_cols(const SolveArgs& g, const LineStrides& ls) {
     return cudaGetLastError();
 }
 template <class Num, int M>
-cudaError_t launch_transposed_cols(const SolveArgs& g) {
+cudaError_t launch_twist_cols(const SolveArgs& g) {
+    k_twist_cols<Num, M, false><<<cols_grid<M>(g.nsys, 32), 64, 0, g.stream>>>(g);
+    return cudaGetLastError();
+}
+template <class Num, int M>
+cudaError_t launch_transposed_cols(const SolveArgs& g, int twisted) {
+    if (twisted) {
+        k_twist_cols<Num, M, true><<<cols_grid<M>(g.nsys, 32), 64, 0, g.stream>>>(g);
+        return cudaGetLastError();
+    }
     const int tpb = cols_threads<M>(g, 1);
     k_transposed_cols<Num, M><<<cols_grid<M>(g.nsys, tpb), tpb, 0, g.stream>>>(g);
     return cudaGetLastError();

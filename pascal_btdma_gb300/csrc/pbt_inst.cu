@@ -39,7 +39,8 @@ template cudaError_t launch_adjoint<PBT_NUM, PBT_M>(const SolveArgs&, const Adjo
 template cudaError_t launch_batch<PBT_NUM, PBT_M>(const BatchArgs&, int, cudaStream_t, int*);
 template cudaError_t launch_thomas_cols<PBT_NUM, PBT_M>(const SolveArgs&, const LineStrides&);
 template cudaError_t launch_modi_cols<PBT_NUM, PBT_M>(const SolveArgs&);
-template cudaError_t launch_transposed_cols<PBT_NUM, PBT_M>(const SolveArgs&);
+template cudaError_t launch_transposed_cols<PBT_NUM, PBT_M>(const SolveArgs&, int);
+template cudaError_t launch_twist_cols<PBT_NUM, PBT_M>(const SolveArgs&);
 template cudaError_t launch_reduced_cols<PBT_NUM, PBT_M>(const SolveArgs&);
 #endif
 #ifdef PBT_HAS_RING

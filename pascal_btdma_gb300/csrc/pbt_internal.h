@@ -88,16 +88,33 @@ template <class Num, int M> cudaError_t launch_modi(const SolveArgs& g);
 template <class Num, int M> cudaError_t launch_reduced(const SolveArgs& g);
 template <class Num, int M> cudaError_t launch_reduced_cyclic(const SolveArgs& g);
 template <class Num, int M> cudaError_t launch_update(const SolveArgs& g);
+// Measured costs of one lane per block column (pbt_cols.cuh) and of the two-stage
+// method, by m = 1 .. 10, from sweeps on a GB300: us a row of a line's chain, ns
+// a row of a batch that fills the GPU, ns a row of the local stage and update of
+// a batch that does not quite.  They decide between methods, so what counts is
+// their order, not the last tenth.
+struct ColsCost {
+    double chain[10], row[10], segmented[10];
+};
+constexpr ColsCost kColsFF = {{1.0, 1.3, 1.45, 2.15, 2.7, 3.3, 5.0, 6.4, 9.0, 11.0},
+                              {0.03, 0.06, 0.12, 0.29, 0.49, 0.87, 1.35, 1.95, 3.0, 4.5},
+                              {0.05, 0.10, 0.33, 0.60, 1.05, 3.5, 4.0, 6.8, 10.0, 14.0}};
+constexpr ColsCost kColsF64 = {{1.0, 1.4, 2.4, 4.2, 5.6, 7.6, 9.3, 12.3, 16.0, 19.0},
+                               {0.08, 0.19, 0.46, 0.96, 1.6, 2.5, 3.9, 6.5, 9.0, 13.0},
+                               {0.10, 0.18, 0.60, 1.14, 2.2, 4.0, 5.5, 8.0, 14.0, 20.0}};
+
 // One lane per block column (pbt_cols.cuh; F64 and FF, m <= kColsMaxBlock),
 // for batches too small for one thread per system: the single-segment solve of
 // lines by strides, the local stage, and the reduced solve.
 constexpr int kColsMaxBlock = PBT_MAX_BLOCK;
 template <class Num, int M> cudaError_t launch_thomas_cols(const SolveArgs& g, const LineStrides& ls);
 template <class Num, int M> cudaError_t launch_modi_cols(const SolveArgs& g);
+// The single-segment solve eliminated from both ends (raw factors in g.cw).
+template <class Num, int M> cudaError_t launch_twist_cols(const SolveArgs& g);
 // M^T x = d for the blocks in a, b, c (x, d in g.d), raw factors in g.cw: one
 // lane a column, and through the CTA's ring (maps.a over C, maps.c over A, with
 // the block's two indices as separate dimensions).
-template <class Num, int M> cudaError_t launch_transposed_cols(const SolveArgs& g);
+template <class Num, int M> cudaError_t launch_transposed_cols(const SolveArgs& g, int twisted);
 template <class Num, int M>
 cudaError_t launch_transposed_ring(const SolveArgs& g, const LineStrides& ls, const ThomasMaps& maps);
 template <class Num, int M> cudaError_t launch_reduced_cols(const SolveArgs& g);
