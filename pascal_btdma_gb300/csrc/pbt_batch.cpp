@@ -285,20 +285,36 @@ int pbt_batch_create(pbt_batch** out, int nsys, const int* m, const int* nrow, i
         by_cost.push_back({total, mm});
     }
     if (cols) {
-        // Longest chain first: the order in which the CTAs start.
+        // CTAs of one block size, its items by decreasing chain; then the
+        // longest chain first, the order in which they start.
         const pbt::ColsCost& c = precision == PBT_PREC_FF ? pbt::kColsFF : pbt::kColsF64;
-        std::vector<It> it1;
-        for (int t = 0; t < b->ntiles; ++t) {
-            const auto& tl = tiles[t];
-            if (!by_cols(tl)) continue;
-            const int per = (32 / (tl.m + 1)) * (tl.nseg > 1 ? 1 : 2);  // systems an item
-            for (int k = 0; k * per < tl.lanes; ++k)
-                it1.push_back({t, k, c.chain[tl.m - 1] * tl.rows / (tl.nseg > 1 ? 2 : 1)});
+        struct Cta {
+            int2 item[pbt::kBatchColsMaxPairs];
+            double cost;
+        };
+        const size_t pairs = (size_t)pbt::batch_cols_pairs(precision == PBT_PREC_FF);
+        std::vector<Cta> ctas;
+        for (int mm = 1; mm <= pbt::kBatchColsMaxBlock; ++mm) {
+            std::vector<It> it1;
+            for (int t = 0; t < b->ntiles; ++t) {
+                const auto& tl = tiles[t];
+                if (tl.m != mm) continue;
+                const int per = (32 / (mm + 1)) * (tl.nseg > 1 ? 1 : 2);  // systems an item
+                for (int k = 0; k * per < tl.lanes; ++k)
+                    it1.push_back({t, k, c.chain[mm - 1] * tl.rows / (tl.nseg > 1 ? 2 : 1)});
+            }
+            std::stable_sort(it1.begin(), it1.end(), [](const It& x, const It& y) { return x.cost > y.cost; });
+            for (size_t i = 0; i < it1.size(); i += pairs) {
+                Cta x{{}, it1[i].cost};
+                for (size_t k = 0; k < pairs; ++k)
+                    x.item[k] = i + k < it1.size() ? make_int2(it1[i + k].t, it1[i + k].s) : make_int2(0, -1);
+                ctas.push_back(x);
+            }
         }
-        std::stable_sort(it1.begin(), it1.end(), [](const It& x, const It& y) { return x.cost > y.cost; });
+        std::stable_sort(ctas.begin(), ctas.end(), [](const Cta& x, const Cta& y) { return x.cost > y.cost; });
         b->off_cols = (int)items1.size();
-        b->cnt_cols = (int)it1.size();
-        for (const auto& i : it1) items1.push_back(make_int2(i.t, i.s));
+        for (const auto& x : ctas) items1.insert(items1.end(), x.item, x.item + pairs);
+        b->cnt_cols = (int)items1.size() - b->off_cols;
     }
     std::stable_sort(by_cost.begin(), by_cost.end(), [](const std::pair<double, int>& x, const std::pair<double, int>& y) {
         return x.first > y.first;
@@ -425,7 +441,7 @@ int pbt_batch_solve(pbt_batch* b, const double* pa, const double* pb, const doub
         ba.head1 = nullptr;
         if ((e = pbt::launch_batch_cols(ba, b->precision == PBT_PREC_FF, s)) != cudaSuccess)
             return bcuda(e, "batch_solve: launch");
-        b->last_grid = b->cnt_cols;
+        b->last_grid = b->cnt_cols / pbt::batch_cols_pairs(b->precision == PBT_PREC_FF);
     }
     for (int mm : b->order) {
         ba.items1 = b->items1 + b->off1[mm];

@@ -10,18 +10,23 @@
 // that the whole batch keeps the GPU busy: block Thomas's arithmetic, every
 // value read once, all block sizes in one launch, longest items first.  The
 // rule is cols_solve (pbt_batch.cpp).  Uneven batch of 32768 systems, N 16 ..
-// 4096, m 2 .. 5, float-float (GB300): 13232 -> 10611 us a solve and unpack.
+// 4096, m 2 .. 5 (GB300), us a solve and unpack: float-float segments 13232, this
+// with one pair of warps a CTA 10710, two 9484, four 8891, eight 10178 -- with
+// pairs of every block size on an SM, their unrolled rows miss the instruction
+// cache (63 % hits, "no instruction" half of all stalls), with eight a CTA waits
+// for its longest; FP64, whose rows are short, 23238, 23616, 25989, 35174.
 #include "pbt_batch_types.h"
 #include "pbt_cols.cuh"
 
 namespace pbt {
 
 // A tile planned in one segment is solved from its first row on, each warp of
-// the CTA a group of its own; one planned in several by both ends (twisted),
-// the CTA's two warps on one group.
+// the pair a group of its own; one planned in several by both ends (twisted),
+// the pair's two warps on one group.
 template <class Num, int M>
-__device__ __forceinline__ void batch_cols(const BatchArgs& ba, const BatchTile& tl, int group, double* sh) {
-    const int side = threadIdx.x >> 5;
+__device__ __forceinline__ void batch_cols(const BatchArgs& ba, const BatchTile& tl, int group, double* sh,
+                                           int bar) {
+    const int side = (threadIdx.x >> 5) & 1;
     const bool twisted = tl.nseg > 1;
     const ColLane cl = col_lane<M>(tl.lanes, twisted ? group : 2 * group + side);
     const int rows = tl.rows, n0 = rows / 2, n = twisted ? (side ? rows - n0 : n0) : rows;
@@ -30,34 +35,39 @@ __device__ __forceinline__ void batch_cols(const BatchArgs& ba, const BatchTile&
     if (twisted)
         thomas_cols_body<Num, M, false, false, true>((side ? ba.c : ba.a) + mo, ba.b + mo, (side ? ba.a : ba.c) + mo,
                                                      ba.d + vo, ba.cw + mo, plane, side ? -32 : 32, n, true, ba.status,
-                                                     cl, side, sh);
+                                                     cl, side, sh, bar);
     else
         thomas_cols_body<Num, M, false>(ba.a + mo, ba.b + mo, ba.c + mo, ba.d + vo, ba.cw + mo, plane, 32, n, true,
                                         ba.status, cl);
 }
 
 template <class Num>
-__global__ void __launch_bounds__(64, 8) k_batch_cols(const BatchArgs ba) {
-    __shared__ double sh[2 * 32 * kBatchColsMaxBlock];
-    const int2 it = ba.items1[blockIdx.x];
+__global__ void __launch_bounds__(64 * batch_cols_pairs(Num::kConv), 8 / batch_cols_pairs(Num::kConv))
+    k_batch_cols(const BatchArgs ba) {
+    constexpr int kPairs = Num::kConv ? kBatchColsMaxPairs : 1;  // batch_cols_pairs
+    __shared__ double sh[kPairs][2 * 32 * kBatchColsMaxBlock];
+    const int pair = threadIdx.x >> 6;
+    const int2 it = ba.items1[blockIdx.x * kPairs + pair];
+    if (it.y < 0) return;  // the last CTA of a block size is not full
     const BatchTile tl = ba.tiles[it.x];
     switch (tl.m) {
-        case 1: batch_cols<Num, 1>(ba, tl, it.y, sh); break;
-        case 2: batch_cols<Num, 2>(ba, tl, it.y, sh); break;
-        case 3: batch_cols<Num, 3>(ba, tl, it.y, sh); break;
-        case 4: batch_cols<Num, 4>(ba, tl, it.y, sh); break;
-        case 5: batch_cols<Num, 5>(ba, tl, it.y, sh); break;
-        default: batch_cols<Num, 6>(ba, tl, it.y, sh); break;
+        case 1: batch_cols<Num, 1>(ba, tl, it.y, sh[pair], 1 + pair); break;
+        case 2: batch_cols<Num, 2>(ba, tl, it.y, sh[pair], 1 + pair); break;
+        case 3: batch_cols<Num, 3>(ba, tl, it.y, sh[pair], 1 + pair); break;
+        case 4: batch_cols<Num, 4>(ba, tl, it.y, sh[pair], 1 + pair); break;
+        case 5: batch_cols<Num, 5>(ba, tl, it.y, sh[pair], 1 + pair); break;
+        default: batch_cols<Num, 6>(ba, tl, it.y, sh[pair], 1 + pair); break;
     }
 }
 static_assert(kBatchColsMaxBlock == 6, "k_batch_cols lists block sizes 1..6");
 
 cudaError_t launch_batch_cols(const BatchArgs& ba, int ff, cudaStream_t s) {
     if (ba.n1 <= 0) return cudaSuccess;
+    const int pairs = batch_cols_pairs(ff != 0);
     if (ff)
-        k_batch_cols<FF><<<(unsigned)ba.n1, 64, 0, s>>>(ba);
+        k_batch_cols<FF><<<(unsigned)(ba.n1 / pairs), 64 * pairs, 0, s>>>(ba);
     else
-        k_batch_cols<F64><<<(unsigned)ba.n1, 64, 0, s>>>(ba);
+        k_batch_cols<F64><<<(unsigned)(ba.n1 / pairs), 64 * pairs, 0, s>>>(ba);
     return cudaGetLastError();
 }
 

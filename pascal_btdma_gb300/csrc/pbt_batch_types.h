@@ -51,9 +51,12 @@ struct PackArgs {
 };
 constexpr int kPackRows = 64;
 
-// Block sizes up to this may be solved by k_batch_cols (pbt_batch_cols.cu):
-// one CTA of two warps per item (tile, group of systems) in items1.
+// Block sizes up to this may be solved by k_batch_cols (pbt_batch_cols.cu): a
+// pair of warps per item (tile, group of systems) in items1, in CTAs of
+// batch_cols_pairs consecutive items of one block size (group -1: none).
 constexpr int kBatchColsMaxBlock = 6;
+constexpr int kBatchColsMaxPairs = 4;
+constexpr int batch_cols_pairs(bool ff) { return ff ? kBatchColsMaxPairs : 1; }
 cudaError_t launch_batch_cols(const BatchArgs& ba, int ff, cudaStream_t s);
 
 // The launches of block size M (pbt_batch.cuh; instantiated with the other

@@ -63,6 +63,9 @@ __device__ __forceinline__ long long grid_warp() {
     return (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
 }
 
+// Barrier `id` of the 64 threads of a pair of warps.
+__device__ __forceinline__ void pair_barrier(int id) { asm volatile("barrier.sync %0, 64;" ::"r"(id) : "memory"); }
+
 // M values `stride` apart at p (zeros on a lane that is not live), raw.
 template <int M>
 __device__ __forceinline__ void col_load(double (&v)[M], const double* p, size_t stride, bool live) {
@@ -214,7 +217,7 @@ template <class Num, int M, bool Reduced, bool Transposed = false, bool Twisted 
 __device__ __forceinline__ void thomas_cols_body(const double* A, const double* B, const double* C, double* D,
                                                  double* CW, size_t plane, ptrdiff_t rs, int N, bool raw,
                                                  unsigned long long* status, const ColLane& cl, int side = 0,
-                                                 double* sh = nullptr) {
+                                                 double* sh = nullptr, int bar = 1) {
     using T = typename Num::T;
     using Acc = typename Num::Acc;
     const bool rhs = cl.j == M;
@@ -283,7 +286,7 @@ __device__ __forceinline__ void thomas_cols_body(const double* A, const double* 
         const double* const other = sh + ((side ^ 1) * 32 + (threadIdx.x & 31)) * M;
 #pragma unroll
         for (int i = 0; i < M; ++i) Num::sts(mine + i, cp[i]);
-        __syncthreads();
+        pair_barrier(bar);
         T oc[M];
         Acc r[M], x[1][M];
 #pragma unroll
@@ -357,12 +360,12 @@ __device__ __forceinline__ void thomas_cols_body(const double* A, const double* 
         // The line's outcome, both sides together, reported by side 0.
         col_merge<M>(bad, amax, cl);
         unsigned* const u = reinterpret_cast<unsigned*>(sh) + 2 * (threadIdx.x & 31);
-        __syncthreads();  // the exchange has been read
+        pair_barrier(bar);  // the exchange has been read
         if (side == 1) {
             u[0] = bad;
             u[1] = amax;
         }
-        __syncthreads();
+        pair_barrier(bar);
         if (side == 0 && cl.live && cl.j == 0)
             report_status(status, bad | u[0] | range_bits<Num>(max(amax, u[1]), true));
     } else {
