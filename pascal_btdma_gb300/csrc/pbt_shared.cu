@@ -45,23 +45,25 @@ constexpr unsigned kSharedMagic = 0x50425453u;
 constexpr int kSharedWarps = 4;
 constexpr int kSharedThreads = 32 * kSharedWarps;
 
-// A warp owns 32 consecutive lines and walks them in chunks of K block rows
-// (K*M <= 16 doubles, 128 bytes of a line).  A chunk is staged in shared
-// memory, [line][K*M] with an odd row stride S (no bank conflicts), by
-// coalesced loads whatever the layout:
-//   contiguous lines (elem_stride 1, row_stride M: the sweep along the fast
-//     axis): each half-warp reads one line's chunk, 128 contiguous bytes;
-//   otherwise: lane = line, one load per element of the chunk, 32 lines
-//     side by side (256 contiguous bytes when stride_inner is 1).
-// Each lane then runs its own line's recurrence on the tile and the tile is
-// written back the same way.  The forward sweep leaves y in x; the last chunk
-// turns around in shared memory, and the backward sweep reloads the other
-// chunks last to first.  Latency is hidden by warps, not by prefetching in a
-// warp: registers are capped so that as many blocks fit on an SM as the
-// arithmetic allows without spills (shared_min_blocks).
-template <int M>
+// Contiguous lines (elem_stride 1, row_stride M: the sweep along the fast axis).
+// A warp owns 32 consecutive lines and walks them in chunks of K block rows, at
+// most P values of a line, staged in shared memory, [line][K*M] with an odd row
+// stride S (no bank conflicts): P lanes read one line's chunk side by side.  Each
+// lane then runs its own line's recurrence on the tile and the tile is written
+// back the same way.  The forward sweep leaves y in x; the last chunk turns
+// around in shared memory, and the backward sweep reloads the other chunks last
+// to first.  Each chunk is copied (cp.async, 8 bytes a lane: the lines need no
+// more alignment than their type's) while the one before it is solved; loads into
+// registers waited for together were 4.8 of 13 cycles an instruction.  P = 8
+// (64 bytes of a line) leaves room for two tiles a warp at the warps the registers
+// allow: lines of 128 rows, 2^25 unknowns in all, m = 2 float-float 336 -> 290 us, with P = 16
+// 341; m = 10 1980 -> 1173.  FP64 of m >= 3 is at its pipe's rate and has less to
+// do around longer chunks (m = 4: 832 us, 840 with P = 8, 824 with 16), and of 6
+// values only one row fits in 8 (638 us, 615 with 16).
+template <class Num, int M>
 struct SharedTile {
-    static constexpr int K = 16 / M > 0 ? 16 / M : 1;
+    static constexpr int P = M <= 2 || (Num::kConv && M <= 8 && M != 6) ? 8 : 16;  // values of a line in a chunk, at most
+    static constexpr int K = P / M > 0 ? P / M : 1;
     static constexpr int KM = K * M;
     static constexpr int S = KM | 1;
 };
@@ -72,81 +74,33 @@ __host__ __device__ constexpr int shared_min_blocks() {
     return Num::kConv ? (M <= 2 ? 8 : M <= 4 ? 6 : 4) : (M <= 4 ? 5 : 4);
 }
 
-// Chunk moves.  fetch() issues a chunk's loads into registers (v: up to 16
-// doubles a lane), deposit() puts them in the tile, store() writes the tile
-// out; a lane's loads all go out before anything waits on them.
-template <int M>
-__device__ __forceinline__ void fetch(const double* src, double* v, long long base, bool live, int nlive, int q0, int kk,
-                                      const pbt_lines& L, bool contiguous) {
-    constexpr int K = SharedTile<M>::K;
-    static_assert(SharedTile<M>::KM <= 16, "a chunk is at most 16 doubles of a line");
-    const int lane = threadIdx.x & 31;
-    if (contiguous) {
-        const int len = kk * M, half = lane >> 4, e = lane & 15;
+// Chunk moves: fetch() starts a chunk's copies into a tile, store() writes the
+// tile out.
+template <class Num, int M>
+__device__ __forceinline__ void fetch(const double* src, double* tile, long long base, int nlive, int q0, int kk) {
+    constexpr int S = SharedTile<Num, M>::S, P = SharedTile<Num, M>::P;
+    const int lane = threadIdx.x & 31, len = kk * M, part = lane / P, e = lane % P;
 #pragma unroll
-        for (int it = 0; it < 16; ++it) {
-            const int j = 2 * it + half;
-            const long long bj = __shfl_sync(0xffffffffu, base, j) + (long long)q0 * M + e;
-            v[it] = (j < nlive && e < len) ? src[bj] : 0.0;
-        }
-    } else if (live) {
-#pragma unroll
-        for (int u = 0; u < K; ++u) {
-            if (u < kk) {
-                const long long r = base + (long long)(q0 + u) * L.row_stride;
-#pragma unroll
-                for (int i = 0; i < M; ++i) v[u * M + i] = src[r + i * L.elem_stride];
-            }
+    for (int it = 0; it < P; ++it) {
+        const int j = 32 / P * it + part;
+        const long long bj = __shfl_sync(0xffffffffu, base, j) + (long long)q0 * M + e;
+        if (j < nlive && e < len) {
+            const unsigned to = (unsigned)__cvta_generic_to_shared(tile + j * S + e);
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(to), "l"(src + bj) : "memory");
         }
     }
 }
 
-template <int M>
-__device__ __forceinline__ void deposit(const double* v, double* tile, bool live, int nlive, int kk, bool contiguous) {
-    constexpr int K = SharedTile<M>::K, S = SharedTile<M>::S;
-    const int lane = threadIdx.x & 31;
-    if (contiguous) {
-        const int len = kk * M, half = lane >> 4, e = lane & 15;
-#pragma unroll
-        for (int it = 0; it < 16; ++it) {
-            const int j = 2 * it + half;
-            if (j < nlive && e < len) tile[j * S + e] = v[it];
-        }
-    } else if (live) {
-        double* my = tile + lane * S;
-#pragma unroll
-        for (int u = 0; u < K; ++u)
-            if (u < kk)
-#pragma unroll
-                for (int i = 0; i < M; ++i) my[u * M + i] = v[u * M + i];
-    }
+template <class Num, int M>
+__device__ __forceinline__ void store(double* dst, const double* tile, long long base, int nlive, int q0, int kk) {
+    constexpr int S = SharedTile<Num, M>::S, P = SharedTile<Num, M>::P;
+    const int lane = threadIdx.x & 31, len = kk * M, part = lane / P, e = lane % P;
     __syncwarp();
-}
-
-template <int M>
-__device__ __forceinline__ void store(double* dst, const double* tile, long long base, bool live, int nlive, int q0,
-                                      int kk, const pbt_lines& L, bool contiguous) {
-    constexpr int K = SharedTile<M>::K, S = SharedTile<M>::S;
-    const int lane = threadIdx.x & 31;
-    __syncwarp();
-    if (contiguous) {
-        const int len = kk * M, half = lane >> 4, e = lane & 15;
 #pragma unroll
-        for (int it = 0; it < 16; ++it) {
-            const int j = 2 * it + half;
-            const long long bj = __shfl_sync(0xffffffffu, base, j) + (long long)q0 * M + e;
-            if (j < nlive && e < len) dst[bj] = tile[j * S + e];
-        }
-    } else if (live) {
-        const double* my = tile + lane * S;
-#pragma unroll
-        for (int u = 0; u < K; ++u) {
-            if (u < kk) {
-                const long long r = base + (long long)(q0 + u) * L.row_stride;
-#pragma unroll
-                for (int i = 0; i < M; ++i) dst[r + i * L.elem_stride] = my[u * M + i];
-            }
-        }
+    for (int it = 0; it < P; ++it) {
+        const int j = 32 / P * it + part;
+        const long long bj = __shfl_sync(0xffffffffu, base, j) + (long long)q0 * M + e;
+        if (j < nlive && e < len) dst[bj] = tile[j * S + e];
     }
     __syncwarp();
 }
@@ -165,52 +119,58 @@ __device__ __forceinline__ pbt::ff ldf<pbt::FF>(const double* p) {
 }
 
 // y = R_q^{-1} (t - A_q y_prev) with the stored factors of R_q (t in, y out).
+// The pivots are the matrix's, the same for every line, so a swap is a branch
+// that the whole warp takes or not (FP64 up to m = 5 selects instead: the branch
+// cost it 0.5 %); the sums stay unnormalised between steps, as in lu_solve, but
+// for one normalisation above m = 6, without which the error against 64 bits grew
+// with m past that of normalised sums (m = 10: 1.24e-14; 1.13e-14 with it, 1.15e-14
+// normalised at every step).
 template <class Num, int M>
 __device__ __forceinline__ void forward_row(const double* __restrict__ fac, const long long* __restrict__ pivs, int q,
-                                            typename Num::T* t, typename Num::T* y) {
+                                            const typename Num::T* t, typename Num::T* y) {
     using T = typename Num::T;
+    using Acc = typename Num::Acc;
     const double* Aq = fac + (size_t)q * 3 * M * M;
     const double* F = Aq + M * M;
     const long long pq = __ldg(pivs + q);
+    Acc a[M];
+#pragma unroll
+    for (int i = 0; i < M; ++i) a[i] = Num::acc(t[i]);
     if (q > 0) {
 #pragma unroll
-        for (int i = 0; i < M; ++i) {
-            typename Num::Acc a = Num::acc(t[i]);
+        for (int i = 0; i < M; ++i)
 #pragma unroll
-            for (int k = 0; k < M; ++k) Num::msub(a, ldf<Num>(Aq + i + M * k), y[k]);
-            t[i] = Num::fin(a);
+            for (int k = 0; k < M; ++k) Num::msub(a[i], ldf<Num>(Aq + i + M * k), y[k]);
+        if (M > 6) {
+#pragma unroll
+            for (int i = 0; i < M; ++i) a[i] = Num::acc(Num::fin(a[i]));
         }
     }
-    // Replay the elimination of R_q on t, then back-substitute.
+    // Replay the elimination of R_q, then back-substitute.
 #pragma unroll
     for (int k = 0; k < M; ++k) {
         if (k + 1 < M) {
             const int p = (int)((pq >> (4 * k)) & 15);
+            if (p != k || (!Num::kConv && M <= 5)) {
 #pragma unroll
-            for (int i = k + 1; i < M; ++i) {
-                const unsigned sw = (p == i);
-                const T a = t[k], b = t[i];
-                t[k] = Num::sel(sw, b, a);
-                t[i] = Num::sel(sw, a, b);
+                for (int i = k + 1; i < M; ++i) {
+                    const unsigned sw = (p == i);
+                    const Acc u = a[k], v = a[i];
+                    a[k] = Num::asel(sw, v, u);
+                    a[i] = Num::asel(sw, u, v);
+                }
             }
         }
+        const T bk = Num::fin(a[k]);
+        a[k] = Num::acc(bk);
 #pragma unroll
-        for (int i = k + 1; i < M; ++i) {
-            typename Num::Acc a = Num::acc(t[i]);
-            Num::msub(a, ldf<Num>(F + i + M * k), t[k]);
-            t[i] = Num::fin(a);
-        }
+        for (int i = k + 1; i < M; ++i) Num::msub(a[i], ldf<Num>(F + i + M * k), bk);
     }
 #pragma unroll
     for (int k = M - 1; k >= 0; --k) {
-        const T xk = Num::mul(t[k], ldf<Num>(F + k + M * k));
-        y[k] = xk;
+        y[k] = Num::mul(Num::fin(a[k]), ldf<Num>(F + k + M * k));
 #pragma unroll
-        for (int i = 0; i < k; ++i) {
-            typename Num::Acc a = Num::acc(t[i]);
-            Num::msub(a, ldf<Num>(F + i + M * k), xk);
-            t[i] = Num::fin(a);
-        }
+        for (int i = 0; i < k; ++i) Num::msub(a[i], ldf<Num>(F + i + M * k), y[k]);
     }
 }
 
@@ -237,22 +197,19 @@ template <class Num, int M>
 __global__ void __launch_bounds__(kSharedThreads, (shared_min_blocks<Num, M>())) k_shared(const double* __restrict__ fac,
                                                            const long long* __restrict__ pivs,
                                                            const double* rhs, double* x, int nrow, pbt_lines L,
-                                                           int contiguous, unsigned long long* status) {
+                                                           unsigned long long* status) {
     using T = typename Num::T;
-    constexpr int K = SharedTile<M>::K, S = SharedTile<M>::S;
-    __shared__ double tiles[kSharedWarps][32 * S];
+    constexpr int K = SharedTile<Num, M>::K, S = SharedTile<Num, M>::S;
+    __shared__ double tiles[kSharedWarps][2][32 * S];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const long long nsys = (long long)L.nsys_inner * L.nsys_outer;
     const long long s0 = ((long long)blockIdx.x * kSharedWarps + w) * 32;
     if (s0 >= nsys) return;  // the whole warp
-    double* tile = tiles[w];
-    double* my = tile + lane * S;
     const long long s = s0 + lane;
     const bool live = s < nsys;
     const int nlive = (int)(nsys - s0 < 32 ? nsys - s0 : 32);
     long long base = 0;
     if (live) base = (s % L.nsys_inner) * L.stride_inner + (s / L.nsys_inner) * L.stride_outer;
-    const bool cont = contiguous != 0;
     const int nchunk = (nrow + K - 1) / K;
     // Steps 0..nchunk-1: forward chunks first to last; then the backward
     // sweep over chunks nchunk-2 down to 0 (the last chunk turns around in
@@ -262,14 +219,24 @@ __global__ void __launch_bounds__(kSharedThreads, (shared_min_blocks<Num, M>()))
 #pragma unroll
     for (int i = 0; i < M; ++i) y[i] = Num::zero();
     unsigned amax = 0;  // largest |x| written, for the range check
+    // Step st's chunk is copied while step st - 1 is solved.  What it reads was
+    // stored in step nchunk - 2 at the latest, before a __syncwarp.
+    auto start = [&](int st) {
+        if (st < nsteps) {
+            const int q0 = (st < nchunk ? st : 2 * nchunk - 2 - st) * K;
+            fetch<Num, M>(st < nchunk ? rhs : x, tiles[w][st & 1], base, nlive, q0, min(K, nrow - q0));
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    start(0);
     for (int st = 0; st < nsteps; ++st) {
         const bool fwd = st < nchunk;
         const int q0 = (fwd ? st : 2 * nchunk - 2 - st) * K, kk = min(K, nrow - q0);
-        {
-            double v[16];
-            fetch<M>(fwd ? rhs : x, v, base, live, nlive, q0, kk, L, cont);
-            deposit<M>(v, tile, live, nlive, kk, cont);
-        }
+        double* const tile = tiles[w][st & 1];
+        double* const my = tile + lane * S;
+        start(st + 1);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncwarp();
         if (live && fwd) {
             const bool last = st == nchunk - 1;
 #pragma unroll
@@ -321,9 +288,103 @@ __global__ void __launch_bounds__(kSharedThreads, (shared_min_blocks<Num, M>()))
                 }
             }
         }
-        store<M>(x, tile, base, live, nlive, q0, kk, L, cont);
+        store<Num, M>(x, tile, base, nlive, q0, kk);
     }
     if (live) pbt::report_status(status, pbt::range_bits<Num>(amax, true));
+}
+
+// Lines whose points are not contiguous (the sweeps across the fast axis): a
+// lane's own line straight through registers, neighbouring lanes on neighbouring
+// lines, no tile (its round trip was 16 of 378 instructions a row).  direct_rows
+// rows at a time, the next ones on their way while these are solved.  Measured as
+// above: m = 2 float-float 333 -> 237 us (64 bytes a row and line: 4.5 TB/s), FP64
+// 565 -> 473, m = 4 float-float 515 -> 341, m = 10 1930 -> 991; FP64 of m = 3, 4
+// and 6 stays at its pipe's rate (586 -> 590, 821 -> 814, 1373 -> 1370 us).  The three
+// sweeps of a 512^3 field (m = 2, float-float) went from 3650 to 2900 us, 4.4 GB each.
+template <class Num, int M>
+__host__ __device__ constexpr int direct_rows() {
+    return M == 3 && !Num::kConv ? 5 : M <= 4 ? 8 / M : 1;  // FP64, m = 3: 615 us with 2 rows
+}
+// Blocks an SM must hold: as k_shared's, one less where two rows in registers spilled.
+template <class Num, int M>
+__host__ __device__ constexpr int direct_min_blocks() {
+    return shared_min_blocks<Num, M>() - (Num::kConv && M >= 6 ? 1 : 0);
+}
+template <class Num, int M>
+__global__ void __launch_bounds__(kSharedThreads, (direct_min_blocks<Num, M>())) k_shared_direct(
+    const double* __restrict__ fac, const long long* __restrict__ pivs, const double* rhs, double* x, int nrow,
+    pbt_lines L, unsigned long long* status) {
+    using T = typename Num::T;
+    constexpr int K = direct_rows<Num, M>();
+    const long long s = (long long)blockIdx.x * kSharedThreads + threadIdx.x;
+    if (s >= (long long)L.nsys_inner * L.nsys_outer) return;
+    const long long base = (s % L.nsys_inner) * L.stride_inner + (s / L.nsys_inner) * L.stride_outer;
+    rhs += base;
+    x += base;
+    // Rows q0 .. q0 + K - 1, those inside the line.
+    auto load = [&](double (&v)[K * M], const double* src, int q0) {
+#pragma unroll
+        for (int u = 0; u < K; ++u) {
+            const double* const r = src + (long long)(q0 + u) * L.row_stride;
+#pragma unroll
+            for (int i = 0; i < M; ++i) v[u * M + i] = (q0 + u >= 0 && q0 + u < nrow) ? r[i * L.elem_stride] : 0.0;
+        }
+    };
+    T y[M];
+#pragma unroll
+    for (int i = 0; i < M; ++i) y[i] = Num::zero();
+    unsigned amax = 0;
+    double v[K * M], w[K * M];
+    load(v, rhs, 0);
+    for (int q0 = 0; q0 < nrow; q0 += K) {
+        if (q0 + K < nrow) load(w, rhs, q0 + K);
+#pragma unroll
+        for (int u = 0; u < K; ++u) {
+            const int q = q0 + u;
+            if (q < nrow) {
+                T t[M];
+#pragma unroll
+                for (int i = 0; i < M; ++i) t[i] = Num::in_rhs(&v[u * M + i]);
+                forward_row<Num, M>(fac, pivs, q, t, y);
+                double* const r = x + (long long)q * L.row_stride;
+                const bool last = q == nrow - 1;  // y of the last row is its solution
+#pragma unroll
+                for (int i = 0; i < M; ++i) {
+                    if (last) {
+                        Num::out(r + i * L.elem_stride, y[i]);
+                        amax = max(amax, Num::mag(y[i]));
+                    } else {
+                        Num::sts(r + i * L.elem_stride, y[i]);
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < K * M; ++i) v[i] = w[i];
+    }
+    load(v, x, nrow - 1 - K);
+    for (int q0 = nrow - 1 - K; q0 > -K; q0 -= K) {
+        if (q0 > 0) load(w, x, q0 - K);
+#pragma unroll
+        for (int u = K - 1; u >= 0; --u) {
+            const int q = q0 + u;
+            if (q >= 0) {
+                T t[M];
+#pragma unroll
+                for (int i = 0; i < M; ++i) t[i] = Num::lds(&v[u * M + i]);
+                backward_row<Num, M>(fac, q, t, y);
+                double* const r = x + (long long)q * L.row_stride;
+#pragma unroll
+                for (int i = 0; i < M; ++i) {
+                    Num::out(r + i * L.elem_stride, y[i]);
+                    amax = max(amax, Num::mag(y[i]));
+                }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < K * M; ++i) v[i] = w[i];
+    }
+    pbt::report_status(status, pbt::range_bits<Num>(amax, true));
 }
 
 template <int M>
@@ -332,13 +393,11 @@ cudaError_t launch_shared(const pbt_shared* sh, const double* rhs, double* x, co
     const long long warps = (nsys + 31) / 32;
     const long long grid = (warps + kSharedWarps - 1) / kSharedWarps;
     if (grid > 0x7fffffffLL) return cudaErrorInvalidValue;
-    const int contiguous = (L.elem_stride == 1 && L.row_stride == M) ? 1 : 0;
-    if (sh->precision == PBT_PREC_FF)
-        k_shared<pbt::FF, M><<<(unsigned)grid, kSharedThreads, 0, st>>>(sh->fac, sh->piv, rhs, x, sh->nrow, L,
-                                                                        contiguous, sh->status);
-    else
-        k_shared<pbt::F64, M><<<(unsigned)grid, kSharedThreads, 0, st>>>(sh->fac, sh->piv, rhs, x, sh->nrow, L,
-                                                                         contiguous, sh->status);
+    const bool ff = sh->precision == PBT_PREC_FF;
+    const auto kernel = (L.elem_stride == 1 && L.row_stride == M)  // contiguous lines
+                            ? (ff ? k_shared<pbt::FF, M> : k_shared<pbt::F64, M>)
+                            : (ff ? k_shared_direct<pbt::FF, M> : k_shared_direct<pbt::F64, M>);
+    kernel<<<(unsigned)grid, kSharedThreads, 0, st>>>(sh->fac, sh->piv, rhs, x, sh->nrow, L, sh->status);
     return cudaGetLastError();
 }
 

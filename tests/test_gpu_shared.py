@@ -105,3 +105,32 @@ def test_contiguous_lines(cuda, m, nrow, nsys, prec):
     got = x.cpu().numpy()
     err = np.abs(got - want).max(axis=(1, 2)) / np.abs(want).max(axis=(1, 2))
     assert err.max() <= TOL
+
+
+@pytest.mark.parametrize("prec", PRECS)
+@pytest.mark.parametrize("m", range(1, 11))
+def test_contiguous_lines_equal_packed_ones(cuda, m, prec):
+    """Lines along the fast axis go through a tile in shared memory, others
+    through registers: the same arithmetic, so the same bits, at line lengths
+    around every chunk's edge (at most 16 values and at most 8 rows), with a
+    last warp that is not full, out of place and in place."""
+    nsys = 70
+    for nrow in sorted({2, 3, 8 // m + 1, 16 // m, 16 // m + 1, 2 * (16 // m) + 1, 9, 25} - {0, 1}):
+        a, b, c = one_system(m, nrow, seed=m)
+        rng = np.random.default_rng(nrow)
+        d = rng.uniform(-1, 1, (nrow, m, nsys))
+        ref = d.transpose(1, 0, 2).reshape(-1).copy()
+        O.solve_noncyclic(m, nsys, nrow, 1, replicate(a, nsys), replicate(b, nsys), replicate(c, nsys), ref)
+        across = torch.from_numpy(d.copy()).to(cuda)  # [row, unknown, line]
+        along = across.permute(2, 0, 1).contiguous()  # [line, row, unknown]
+        out = torch.empty_like(along)
+        with shared.SharedMatrix(m, nrow, a, b, c, precision=prec) as sm:
+            lines = shared.Lines(nsys, 1, nrow * m, 0, m, 1)
+            sm.solve(along, out, lines)
+            sm.solve(along, along, lines)
+            sm.solve(across, across, shared.Lines(nsys, 1, 1, 0, m * nsys, nsys))
+            torch.cuda.synchronize()
+        assert torch.equal(out, along)
+        assert torch.equal(across.permute(2, 0, 1), out)
+        got = across.permute(1, 0, 2).cpu().numpy().reshape(-1)
+        assert per_system_relerr(m, nsys, nrow, got, ref) <= TOL
