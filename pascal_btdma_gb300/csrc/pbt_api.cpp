@@ -357,12 +357,12 @@ cudaError_t run_reduced_cols(int arith, int m, const pbt::SolveArgs& g) {
 // item, whose threads per SM they would be; the bits are the same.  From
 // sweeps on GB300 (152 SMs; us, one thread -> one lane a column, on both sides
 // of the line):
-//   FP64, line at 70 threads an SM (10640 systems x 64 rows), 90 for m <= 3 and
-//     the local stage: m = 3 12288 425 -> 371, 16384 441 -> 485; m = 5 1024
-//     1236 -> 361, 10240 1249 -> 1109, 12288 1249 -> 1443; m = 8 10240 4090 ->
-//     3829, 12288 4108 -> 5626; m = 10 4096 7986 -> 3999, 8192 7985 -> 8464
-//     (line at 45); local stage 3, 1024 x 128 in 4 342 -> 176,
-//     4, 2048 x 512 in 8 1567 -> 1761;
+//   FP64, line at 90 threads an SM up to m = 3 (13680 systems) and for the local
+//     stage, 60 to 84 above (against the CTA's ring for m = 4 to 6): 64 rows, m = 3
+//     12288 425 -> 371, 16384 441 -> 485; 128 rows, m = 4 11400 1370 -> 1294; m =
+//     5 11800 2276 -> 2228; m = 6 13000 3720 -> 4220; m = 7 10400 6027 -> 4809; m
+//     = 8 10400 8170 -> 7870; m = 10 7600 16146 -> 13753, 9000 16119 -> 14550;
+//     local stage 3, 1024 x 128 in 4 342 -> 176, 4, 2048 x 512 in 8 1567 -> 1761;
 //   float-float, line at 180 (27360), 384 for m <= 3: m = 3 16384 373 -> 170,
 //     65536 534 -> 514; m = 5 4096 723 -> 230, 24000 850 -> 781, 32768 913 ->
 //     1049; m = 8 24000 3295 -> 3002, 32768 3403 -> 4157; local stage 5,
@@ -371,7 +371,8 @@ cudaError_t run_reduced_cols(int arith, int m, const pbt::SolveArgs& g) {
 // multiply-adds in idle slots count from then on.
 bool cols_pay(int arith, int m, long long items, bool local, int sms) {
     if (arith == kF32 || m > pbt::kColsMaxBlock) return false;
-    const int line = arith == kFF ? (!local && m <= 3 ? 384 : 180) : (local || m <= 3 ? 90 : m <= 9 ? 70 : 45);
+    static const int fp64[] = {90, 90, 90, 78, 80, 70, 84, 70, 70, 60};
+    const int line = arith == kFF ? (!local && m <= 3 ? 384 : 180) : (local ? 90 : fp64[m - 1]);
     return items < (long long)line * (sms > 0 ? sms : 1);
 }
 bool thomas_cols(const pbt_plan* p, int arith, int m) {

@@ -378,8 +378,13 @@ template <int M>
 __host__ __device__ constexpr int cols_min_ctas(bool local_stage) {
     return M <= (local_stage ? 4 : 6) ? 4 : (local_stage && M > 6 ? 2 : 3);
 }
+// Warps an SM holds of the single-segment kernels.
+template <int M>
+__host__ __device__ constexpr int cols_warps() {
+    return 4 * cols_min_ctas<M>(false);
+}
 template <class Num, int M>
-__global__ void __launch_bounds__(128, cols_min_ctas<M>(false)) k_thomas_cols(const SolveArgs g, const LineStrides ls) {
+__global__ void __launch_bounds__(32 * cols_warps<M>(), 1) k_thomas_cols(const SolveArgs g, const LineStrides ls) {
     const ColLane cl = col_lane<M>(g.nsys, grid_warp());
     const long long s = cl.live ? cl.sys : 0;
     const size_t o = (size_t)(s % ls.lin) * (size_t)ls.in + (size_t)(s / ls.lin) * (size_t)ls.out;
@@ -399,7 +404,7 @@ __global__ void __launch_bounds__(128, cols_min_ctas<M>(false)) k_reduced_cols(c
 // At_q = C_{q-1}^T, Bt_q = B_q^T, Ct_q = A_{q+1}^T; lambda in D, the factors in
 // the workspace (raw).
 template <class Num, int M>
-__global__ void __launch_bounds__(128, cols_min_ctas<M>(false)) k_transposed_cols(const SolveArgs g) {
+__global__ void __launch_bounds__(32 * cols_warps<M>(), 1) k_transposed_cols(const SolveArgs g) {
     const ColLane cl = col_lane<M>(g.nsys, grid_warp());
     const size_t s = cl.live ? (size_t)cl.sys : 0, rs = (size_t)g.nsys;
     thomas_cols_body<Num, M, false, true>(g.c + s - rs, g.b + s, g.a + s + rs, g.d + s, g.cw + s, rs * g.nrow, rs,
@@ -544,14 +549,32 @@ __global__ void __launch_bounds__(128, cols_min_ctas<M>(true)) k_modi_cols(const
     col_report<Num, M>(g.status, bad, 0u, false, cl);
 }
 
-// CTA of the column kernels: one warp while there are fewer than eight warps
-// an SM (they spread over the SMs), else four, whose neighbouring systems
-// share their 32-byte sectors in L1.
+// CTA of the local stage and the reduced solve: one warp while there are fewer
+// than eight warps an SM (they spread over the SMs), else four, whose
+// neighbouring systems share their 32-byte sectors in L1.
 template <int M>
 inline int cols_threads(const SolveArgs& g, int segs) {
     if (!g.tpb_auto) return g.tpb;
     const long long warps = ((long long)g.nsys + cols_systems<M>() - 1) / cols_systems<M>() * segs;
     return warps < 8LL * (g.sms > 0 ? g.sms : 1) ? 32 : 128;
+}
+// CTA of the single-segment kernels: an SM's even share of the warps, or of a
+// round of them where they are not resident together, so that no SM runs longer
+// than another.  In CTAs of four, nine warps an SM made twelve on some, and past
+// residency the first SMs to finish took the rest of the batch between them.
+// FP64, 128 rows: m = 8, 9 warps an SM (4104 systems) 3840 -> 3080 us, 12.5
+// (5700) 7480 -> 4550, 17 7540 -> 6140; m = 5, 9 1675 -> 1358, 12.5 2212 ->
+// 1887.  Float-float up to m = 5 in one round: 7 warps 443 -> 424, 12.5 771 ->
+// 695; its blocks past m = 5 (m = 8, 10 warps 1294 -> 1321) and further rounds
+// (m = 5, 17 warps 984 -> 1017) are better off in fours, whose code and sectors
+// stay in L1 while the fours take turns.
+template <class Num, int M>
+inline int cols_threads_even(const SolveArgs& g) {
+    if (!g.tpb_auto) return g.tpb;
+    const long long n = g.sms > 0 ? g.sms : 1, warps = ((long long)g.nsys + cols_systems<M>() - 1) / cols_systems<M>();
+    const long long even = (warps + n - 1) / n, rounds = (even + cols_warps<M>() - 1) / cols_warps<M>();
+    if (Num::kConv && (M > 5 || rounds > 1)) return cols_threads<M>(g, 1);
+    return 32 * (int)((even + rounds - 1) / rounds);
 }
 template <int M>
 inline unsigned cols_grid(int nsys, int tpb) {
@@ -561,7 +584,7 @@ inline unsigned cols_grid(int nsys, int tpb) {
 
 template <class Num, int M>
 cudaError_t launch_thomas_cols(const SolveArgs& g, const LineStrides& ls) {
-    const int tpb = cols_threads<M>(g, 1);
+    const int tpb = cols_threads_even<Num, M>(g);
     k_thomas_cols<Num, M><<<cols_grid<M>(g.nsys, tpb), tpb, 0, g.stream>>>(g, ls);
     return cudaGetLastError();
 }
@@ -576,7 +599,7 @@ cudaError_t launch_transposed_cols(const SolveArgs& g, int twisted) {
         k_twist_cols<Num, M, true><<<cols_grid<M>(g.nsys, 32), 64, 0, g.stream>>>(g);
         return cudaGetLastError();
     }
-    const int tpb = cols_threads<M>(g, 1);
+    const int tpb = cols_threads_even<Num, M>(g);
     k_transposed_cols<Num, M><<<cols_grid<M>(g.nsys, tpb), tpb, 0, g.stream>>>(g);
     return cudaGetLastError();
 }

@@ -48,6 +48,20 @@ def test_columns_give_the_bits_of_one_thread(cuda, m, prec, warps, extra, nrow, 
         assert np.array_equal(u, v)
 
 
+@pytest.mark.parametrize("m,per_sm", [(1, 5), (3, 11), (5, 7), (5, 16), (6, 17), (7, 11), (8, 13), (10, 12), (10, 25)])
+@pytest.mark.parametrize("prec", ["fp64", "ff"])
+def test_columns_with_an_even_share_of_warps_a_cta(cuda, m, per_sm, prec):
+    """per_sm warps an SM and one less: CTAs of one SM's share, of a round's
+    share past residency (12 warps, 16 up to m = 6), or of four."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    for nsys in (32 // (m + 1) * per_sm * sms, 32 // (m + 1) * (per_sm * sms - sms // 2) - 1):
+        w = synth.dominant(m, nsys, 3, seed=m, delta=1.1)
+        (x, sx), (y, sy) = both(w, cuda, prec)
+        assert sx == sy == 0
+        for u, v in zip(x, y):
+            assert np.array_equal(u, v)
+
+
 @pytest.mark.parametrize("prec", ["fp64", "ff"])
 def test_columns_pivot_and_report_like_one_thread(cuda, prec):
     m, nsys, nrow = 4, 21, 6
