@@ -682,7 +682,7 @@ def run_ours(args):
         vrows = vns * vn
         fills = vns >= 128 * torch.cuda.get_device_properties(dev).multi_processor_count
         entry = {"m": vm, "nsys": vns, "nrow": vn, "nseg": vp, "cyclic": vcyc,
-                 "default_plan_solves_as": (f"{vp} segments" if vp > 1 and not fills else "one segment per line"),
+                 "default_plan_solves_as": (f"{vp} segments or one, by size" if vp > 1 and not fills else "one segment per line"),
                  "l2": "flushed before each solve" if vrows * bytes_per_row(vm) < L2_FIT_BYTES else "inputs > L2"}
         xs = {}
         # With nseg > 1 a batch that fills the GPU is solved one segment per
@@ -733,7 +733,7 @@ def run_ours(args):
         for nseg_m in segs:
             fills = NSYS >= 128 * torch.cuda.get_device_properties(dev).multi_processor_count
             entry = {"delta": delta, "nseg": nseg_m, "row_scale": "log-uniform [1e-3, 1e3]",
-                     "default_plan_solves_as": (f"{nseg_m} segments" if nseg_m > 1 and not fills
+                     "default_plan_solves_as": (f"{nseg_m} segments or one, by size" if nseg_m > 1 and not fills
                                                 else "one segment per line")}
             ref = md.clone()
             with pbt.BtdmaGpuPlan() as p64:

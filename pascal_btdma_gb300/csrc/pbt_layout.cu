@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(kThreads) k_layout(const double* __restrict__ 
 
 // In place: raw float-float pairs (8-byte slots, as the kernels keep their
 // intermediates) <-> FP64 values.  The pair (h, l) has |l| <= ulp(h)/2, so
-// h + l is exact in FP64; back, FF::split_wide keeps 47 bits (these are the
+// h + l is exact in FP64; back, FF::split_wide keeps 47 bits or more (the
 // library's own intermediates: no input window).
 // to_f64 = 2 also sets values below the float-float input window (|v| <
 // 2^-96) to zero: used on the reduced system's blocks before a float-float
