@@ -606,6 +606,11 @@ int kernel_regs(K* k) {
     return a.numRegs > 0 ? a.numRegs : 255;
 }
 
+inline int in_step_cap(size_t smem_thread, int regs) {
+    int cap = 256;
+    while (cap > 32 && (2 * ((size_t)cap * smem_thread + 1024) > 228u * 1024u || 2L * cap * regs > 65536L)) cap -= 32;
+    return cap;
+}
 // CTA size of the in-step kernels: up to 256 threads, as many as two CTAs an
 // SM allow with `smem_thread` bytes of shared memory and `regs` registers a
 // thread, reduced so
@@ -614,13 +619,37 @@ int kernel_regs(K* k) {
 // the caller (threads_per_block) is kept.
 inline int in_step_tpb(const SolveArgs& g, long long units, size_t smem_thread, int regs) {
     if (!g.tpb_auto) return g.tpb;
-    int cap = 256;
-    while (cap > 32 && (2 * ((size_t)cap * smem_thread + 1024) > 228u * 1024u || 2L * cap * regs > 65536L)) cap -= 32;
+    const int cap = in_step_cap(smem_thread, regs);
     const long long sms = g.sms > 0 ? g.sms : 1;
     const long long waves = (units + cap * sms - 1) / (cap * sms);
     long long tpb = (units + waves * sms - 1) / (waves * sms);
     tpb = (tpb + 31) / 32 * 32;
     return (int)(tpb < 32 ? 32 : (tpb > cap ? cap : tpb));
+}
+
+// CTA size of the local stage, whose CTAs stay within a segment: `tpb`, the size
+// for its threads as one row of them, unless the SM with the most warps then
+// has over `slack` percent more of them than with the best size up to `cap`; then
+// the largest size that has not.  Only while all warps are resident: past that
+// the SMs take turns anyway.  256 systems in 224-thread CTAs were two a segment,
+// of 224 and 32 threads.  us, `tpb` -> this: 256 x 32768 in 128 segments,
+// float-float m = 2 1366 -> 1061, m = 4 4104 -> 4009, m = 5 13153 -> 10562 (in
+// step, so larger CTAs are worth up to 20 % of spread: 16384 rows, m = 6 9889
+// with 128 threads, 11588 with 32); FP64 m = 4 8893 -> 7968, m = 5 17108 ->
+// 15388; 1000 x 8192 in 64, m = 5 10821 -> 7630; past residency, 5000 x 2048 in
+// 16, m = 5, 11371 with tpb, 11998 with 32.
+inline int segment_tpb(const SolveArgs& g, int tpb, int cap, int regs, int slack) {
+    if (!g.tpb_auto) return tpb;
+    const long long sms = g.sms > 0 ? g.sms : 1;
+    const auto load = [&](long long t) { return ((g.nsys + t - 1) / t * g.nseg + sms - 1) / sms * (t / 32); };
+    if (((g.nsys + 31LL) / 32 * g.nseg + sms - 1) / sms * 32 * regs > 65536) return tpb;
+    long long best = load(tpb);
+    for (int t = 32; t <= cap; t += 32) best = load(t) < best ? load(t) : best;
+    const auto fits = [&](int t) { return load(t) * 100 <= best * (100 + slack); };
+    if (fits(tpb)) return tpb;
+    for (int t = cap; t > 32; t -= 32)
+        if (fits(t)) return t;
+    return 32;
 }
 
 template <int M>
@@ -2804,8 +2833,10 @@ cudaError_t launch_modi(const SolveArgs& g) {
     if constexpr (modi_uses_lu<Num, M>()) {
         constexpr size_t kSmemThread = cyclic_slots<Num, M>() * sizeof(double);
         static const int regs = kernel_regs(k_modi_lu<Num, M>);
-        const int tpb = rows_in_step<Num>() ? in_step_tpb(g, (long long)g.nsys * g.nseg, kSmemThread, regs)
-                                            : (g.tpb < kThomasThreads ? g.tpb : kThomasThreads);
+        constexpr bool kStep = rows_in_step<Num>();
+        const int one = kStep ? in_step_tpb(g, (long long)g.nsys * g.nseg, kSmemThread, regs)
+                              : (g.tpb < kThomasThreads ? g.tpb : kThomasThreads);
+        const int tpb = segment_tpb(g, one, kStep ? in_step_cap(kSmemThread, regs) : one, regs, kStep ? 20 : 5);
         const size_t smem = (size_t)tpb * kSmemThread;
         if (smem > 48u * 1024u) {
             const cudaError_t e =
@@ -2816,7 +2847,9 @@ cudaError_t launch_modi(const SolveArgs& g) {
         k_modi_lu<Num, M><<<grid, tpb, smem, g.stream>>>(g);
     } else {
         static const int regs = kernel_regs(k_modi<Num, M>);
-        const int tpb = modi_in_step<Num, M>() ? in_step_tpb(g, (long long)g.nsys * g.nseg, 0, regs) : g.tpb;
+        constexpr bool kStep = modi_in_step<Num, M>();
+        const int one = kStep ? in_step_tpb(g, (long long)g.nsys * g.nseg, 0, regs) : g.tpb;
+        const int tpb = segment_tpb(g, one, kStep ? in_step_cap(0, regs) : one, regs, 5);
         dim3 grid(grid_x(g.nsys, tpb), (unsigned)g.nseg);
         k_modi<Num, M><<<grid, tpb, 0, g.stream>>>(g);
     }
