@@ -160,9 +160,11 @@ struct FF {
         const unsigned hb = (__funnelshift_l(lo, hi - (896u << 20), 3) & 0x7fffffffu) | (hi & 0x80000000u);
         unsigned h = (mag2 - (lo_e << 21) < ((hi_e - lo_e + 1u) << 21)) ? hb : 0x7fc00000u;
         h = (mag2 < (zero_e << 21)) ? 0u : h;
-        // Sign and power of two of h (0 for zero, Inf for NaN) times the bits below it.
-        const float l = __fmul_rn(__uint2float_rn(lo & 0x1fffffffu), __uint_as_float(h & 0xff800000u));
-        return {__uint_as_float(h), __fmul_rn(l, 0x1p-52f)};
+        // The bits below h, as a fraction of its power of two (2^-23 at most, so
+        // that the product cannot overflow where h does not), times sign and power
+        // of two of h (0 for zero, Inf for NaN).
+        const float l = __fmul_rn(__uint2float_rn(lo & 0x1fffffffu), 0x1p-52f);
+        return {__uint_as_float(h), __fmul_rn(l, __uint_as_float(h & 0xff800000u))};
     }
 
     // float -> double by bit manipulation: normal floats exactly, Inf and NaN

@@ -170,3 +170,50 @@ def test_batch_and_shared_report(cuda):
         sm.solve(bad)
         with pytest.raises(pbt.ArithmeticRangeError):
             sm.status()
+
+
+@pytest.mark.parametrize("m,nsys,nrow,nseg", [(4, 40, 30, 1), (4, 40, 30, 3), (5, 30000, 4, 1), (3, 60000, 4, 1), (8, 9, 12, 1)])
+def test_large_right_hand_sides_with_full_mantissas(cuda, m, nsys, nrow, nseg):
+    """Right-hand sides up to 2^128 have a low word below 2^105 and are in range,
+    whatever their last bits."""
+    base = synth.dominant(m, nsys, nrow, seed=17, delta=1.5)
+    for val in (1.1e30, -3.3e31, 1.1 * 2.0 ** 120, 1.1 * 2.0 ** 126):
+        w = base.copy()
+        w.D[7 + nsys * (nrow // 2)] = val
+        reported_or_right(w, nseg, "ff", expect_failure=False)
+        w.D[:] *= 2.0 ** 90  # a whole line that large, the rest of the batch inside the window
+        w.D[7 + nsys * (nrow // 2)] = val
+        reported_or_right(w, nseg, "ff", expect_failure=False)
+
+
+def test_large_values_in_place_adjoint_shared_and_long_lines(cuda):
+    w = synth.dominant(3, 50, 24, seed=4, delta=1.5)
+    w.D *= 1.1 * 2.0 ** 115
+    reported_or_right(w, 4, "ff", expect_failure=False, inplace=True)
+    a, b, c, d = to_dev(synth.dominant(3, 50, 24, seed=4, delta=1.5).arrays, cuda)
+    with pbt.BtdmaGpuPlan() as plan:
+        plan.create(3, 50, 24, 1, precision="ff")
+        pbt.solve_noncyclic(plan, a, b, c, d, 3, 50, 24)
+        g = torch.full_like(d, 1.1 * 2.0 ** 115)
+        pbt.adjoint_noncyclic(plan, a, b, c, d, g)
+        assert plan.status() == 0 and bool(torch.isfinite(g).all())
+    m, n = 2, 16
+    w = synth.dominant(m, 1, n, seed=5, delta=1.5)
+    rhs = torch.from_numpy(np.random.default_rng(0).uniform(-1, 1, 33 * n * m)).to(cuda)
+    rhs[40] = 1.1 * 2.0 ** 120
+    x = {}
+    for prec in ("fp64", "ff"):
+        with shared.SharedMatrix(m, n, w.A, w.B, w.C, precision=prec) as sm:
+            x[prec] = rhs.clone()
+            sm.solve(x[prec])
+            sm.status()
+    # lines of n*m contiguous values
+    u, v = (t.view(33, n * m) for t in (x["fp64"], x["ff"]))
+    assert float(((u - v).abs().amax(1) / u.abs().amax(1)).max()) <= TOL["ff"]
+    # Few long lines: the reduced system has a plan of its own, which reads and
+    # writes the reduced solution as FP64.  Inputs inside the window, x near 2^110.
+    w = synth.dominant(4, 16, 4096, seed=6, delta=1.5)
+    for X in (w.A, w.B, w.C):
+        X *= 2.0 ** -40
+    w.D *= 1.1 * 2.0 ** 72
+    reported_or_right(w, 256, "ff", expect_failure=False)
