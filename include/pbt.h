@@ -157,11 +157,18 @@ void pbt_plan_desc_init(pbt_plan_desc* desc);
  * the GPU with one thread per system (nsys >= 128 * SMs, 19456 on a GB300)
  * is solved one segment per line whatever nseg says: the single-segment
  * method does ~40 % of the two-stage method's arithmetic and gives the same x
- * to rounding.  Smaller non-cyclic FP64 and PBT_PREC_FF batches that are not in
+ * to rounding (for lines that block Thomas can solve: every R_q regular).  Smaller non-cyclic FP64 and PBT_PREC_FF batches that are not in
  * place are solved in one segment, or by elimination from both ends of the line
- * at once, where that is faster (same x to rounding).
- * PBT_FLAG_REFERENCE_METHOD keeps the nseg segments (and the reference's
- * in-place A', C' with PBT_FLAG_INPLACE). */
+ * at once, where that is faster.  Those orders of elimination invert other blocks
+ * than the nseg segments do, so a line that they do not suit -- they meet a zero
+ * pivot, or an element of C'_q = R_q^{-1} C_q (from the last row on, of R_q^{-1}
+ * A_q) above 2^10; a singular or tiny last block is an example -- is solved again
+ * in its segments, with their x and their report.  Block diagonally dominant lines
+ * never are; a batch most of whose lines are is solved faster with
+ * PBT_FLAG_REFERENCE_METHOD.  The workspace is that of the segments.
+ * That flag keeps the nseg segments (and the reference's in-place A', C' with
+ * PBT_FLAG_INPLACE), PBT_FLAG_DIRECT_LOADS and PBT_FLAG_STAGED_LOADS keep them on
+ * a batch that does not fill the GPU. */
 int pbt_plan_create(pbt_plan** plan, int m, int nsys, int nrow, int nseg);
 
 /* As pbt_plan_create with every option of pbt_plan_desc. */
@@ -186,8 +193,8 @@ int pbt_solve_noncyclic(pbt_plan* plan, double* a, double* b, double* c, double*
  * btdma_many_mpi_gpu_v2_profiled (mod_btdma_gpu_v2.f90:169-198).  `timings`
  * may be NULL.  Synchronises `stream`.  On a batch below 128 * SMs systems the
  * nseg > 1 segments are solved as such, for their phases, also where
- * pbt_solve_noncyclic would not keep them (the first such call allocates
- * their workspace). */
+ * pbt_solve_noncyclic would not keep them: `total` is then the time of the
+ * segments, not of pbt_solve_noncyclic. */
 int pbt_solve_noncyclic_profiled(pbt_plan* plan, double* a, double* b, double* c, double* d,
                                  int m, int nsys, int nrow, pbt_timings* timings, void* stream);
 

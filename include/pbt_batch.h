@@ -18,7 +18,9 @@
  *
  * Where the batch is large enough for its longest line, the block sizes up to 6
  * are solved in one launch with one lane per block column, lines of several
- * segments by elimination from both ends instead.  Otherwise, and for the
+ * segments by elimination from both ends instead; a line of several segments that
+ * this does not suit (pbt_plan_create tells when) is solved again in them by a
+ * second launch.  Otherwise, and for the
  * larger block sizes, the solve runs, per block size present (largest total
  * cost first), a persistent launch over the local-stage items (the warp that
  * completes a tile's last segment also solves the tile's reduced system) and a
@@ -78,8 +80,8 @@ int pbt_batch_pack(pbt_batch* batch, const double* ua, const double* ub, const d
 int pbt_batch_unpack(pbt_batch* batch, const double* pd, double* ud, void* stream);
 
 /* Solve every system of the batch in place on packed arrays: one memset of
- * the queue state and one launch, or up to two per block size present, no host
- * synchronisation. */
+ * the queue state and up to two launches, or up to two per block size present, no
+ * host synchronisation. */
 int pbt_batch_solve(pbt_batch* batch, const double* pa, const double* pb, const double* pc, double* pd,
                     void* stream);
 

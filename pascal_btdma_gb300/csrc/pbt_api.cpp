@@ -49,6 +49,7 @@ struct pbt_plan {
     bool thomas = false;  // single-segment plain block Thomas path
     bool twisted = false;  // thomas, eliminated from both ends (nseg > 1 only)
     bool lines = false;   // strided lines and the fused adjoint: nseg = 1, or a batch that fills the GPU
+    bool guarded = false;  // thomas by the library's choice for nseg > 1: lines that it does not suit are redone
     bool cyclic_thomas = false;  // single-segment periodic block Thomas (k_thomas_cyclic)
     double* aw = nullptr;  // factor workspace (nullptr when in place)
     double* cw = nullptr;
@@ -57,6 +58,7 @@ struct pbt_plan {
     double* rd = nullptr;
     double* re = nullptr;  // cyclic fill-in column: reduced rows, or every row (cyclic_thomas)
     unsigned long long* status = nullptr;
+    unsigned char* redo = nullptr;  // guarded: a flag a system, clear between solves
     // Iterative refinement (PBT_PREC_FP32_REFINE): iterate X, correction /
     // residual E, convergence statistic, and the outcome of the last solve.
     double* rx = nullptr;
@@ -321,23 +323,29 @@ bool thomas_stages(const pbt_plan* p, int arith, int m, const pbt::SolveArgs& g,
                           : encode_columns(&maps->w, g.cw, g.nsys, g.nrow, mm, m));
 }
 
-cudaError_t run_thomas_cols(int arith, int m, const pbt::SolveArgs& g, const pbt::LineStrides& ls) {
+cudaError_t run_thomas_cols(const pbt_plan* p, int arith, int m, const pbt::SolveArgs& g, const pbt::LineStrides& ls) {
     if (arith == kFF) {
-        PBT_DISPATCH_PLAIN_M2(pbt::FF, launch_thomas_cols, g, ls)
+        PBT_DISPATCH_PLAIN_M2(pbt::FF, launch_thomas_cols, g, ls, p->redo)
     }
-    PBT_DISPATCH_PLAIN_M2(pbt::F64, launch_thomas_cols, g, ls)
+    PBT_DISPATCH_PLAIN_M2(pbt::F64, launch_thomas_cols, g, ls, p->redo)
 }
-cudaError_t run_twist_cols(int arith, int m, const pbt::SolveArgs& g) {
+cudaError_t run_twist_cols(const pbt_plan* p, int arith, int m, const pbt::SolveArgs& g) {
     if (arith == kFF) {
-        PBT_DISPATCH_PLAIN_M2(pbt::FF, launch_twist_cols, g)
+        PBT_DISPATCH_PLAIN_M2(pbt::FF, launch_twist_cols, g, p->redo)
     }
-    PBT_DISPATCH_PLAIN_M2(pbt::F64, launch_twist_cols, g)
+    PBT_DISPATCH_PLAIN_M2(pbt::F64, launch_twist_cols, g, p->redo)
 }
-cudaError_t run_transposed_cols(int arith, int m, const pbt::SolveArgs& g, int twisted) {
+cudaError_t run_transposed_cols(const pbt_plan* p, int arith, int m, const pbt::SolveArgs& g, int twisted) {
     if (arith == kFF) {
-        PBT_DISPATCH_PLAIN_M2(pbt::FF, launch_transposed_cols, g, twisted)
+        PBT_DISPATCH_PLAIN_M2(pbt::FF, launch_transposed_cols, g, twisted, p->redo)
     }
-    PBT_DISPATCH_PLAIN_M2(pbt::F64, launch_transposed_cols, g, twisted)
+    PBT_DISPATCH_PLAIN_M2(pbt::F64, launch_transposed_cols, g, twisted, p->redo)
+}
+cudaError_t run_redo_cols(const pbt_plan* p, int arith, int m, const pbt::SolveArgs& g, int transposed, bool saved) {
+    if (arith == kFF) {
+        PBT_DISPATCH_PLAIN_M2(pbt::FF, launch_redo_cols, g, transposed, p->redo, saved)
+    }
+    PBT_DISPATCH_PLAIN_M2(pbt::F64, launch_redo_cols, g, transposed, p->redo, saved)
 }
 cudaError_t run_modi_cols(int arith, int m, const pbt::SolveArgs& g) {
     if (arith == kFF) {
@@ -435,13 +443,14 @@ bool ring_launch(const pbt_plan* p, int arith, int m, const pbt::SolveArgs& g, c
         !encode_lines(&maps.w, g.cw, g.nsys, g.nrow, ls, mm, m, &rf))
         return false;
     if (arith == kFF)
-        *e = m == 3 ? pbt::launch_thomas_ring<pbt::FF, 3>(g, ls, maps, rf) : pbt::launch_thomas_ring<pbt::FF, 4>(g, ls, maps, rf);
+        *e = m == 3 ? pbt::launch_thomas_ring<pbt::FF, 3>(g, ls, maps, rf, p->redo)
+                    : pbt::launch_thomas_ring<pbt::FF, 4>(g, ls, maps, rf, p->redo);
     else
         switch (m) {
-            case 3: *e = pbt::launch_thomas_ring<pbt::F64, 3>(g, ls, maps, rf); break;
-            case 4: *e = pbt::launch_thomas_ring<pbt::F64, 4>(g, ls, maps, rf); break;
-            case 5: *e = pbt::launch_thomas_ring<pbt::F64, 5>(g, ls, maps, rf); break;
-            default: *e = pbt::launch_thomas_ring<pbt::F64, 6>(g, ls, maps, rf); break;
+            case 3: *e = pbt::launch_thomas_ring<pbt::F64, 3>(g, ls, maps, rf, p->redo); break;
+            case 4: *e = pbt::launch_thomas_ring<pbt::F64, 4>(g, ls, maps, rf, p->redo); break;
+            case 5: *e = pbt::launch_thomas_ring<pbt::F64, 5>(g, ls, maps, rf, p->redo); break;
+            default: *e = pbt::launch_thomas_ring<pbt::F64, 6>(g, ls, maps, rf, p->redo); break;
         }
     return *e != cudaErrorNotSupported;
 }
@@ -462,14 +471,9 @@ bool encode_block_rows(CUtensorMap* tm, const double* base, int nsys, int nrow, 
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// M^T lambda = g (in g.d) of a single-segment plan, straight from the stored
-// blocks: by column lanes or through the ring where the forward solve takes
-// them; false: neither, not launched.
-bool transposed_launch(const pbt_plan* p, int arith, int m, const pbt::SolveArgs& g, cudaError_t* e) {
-    if (p->twisted || thomas_cols(p, arith, m)) {
-        *e = run_transposed_cols(arith, m, g, p->twisted);
-        return true;
-    }
+// M^T x = d through the ring, straight from the stored blocks, where the rule and
+// the tensor maps allow; false: not launched.
+bool transposed_ring(const pbt_plan* p, int arith, int m, const pbt::SolveArgs& g, cudaError_t* e) {
     if (!g.tpb_auto || (p->desc.flags & (PBT_FLAG_DIRECT_LOADS | PBT_FLAG_STAGED_LOADS)) ||
         !prefer_ring(arith, m, g.nsys, p->sms))
         return false;
@@ -483,22 +487,45 @@ bool transposed_launch(const pbt_plan* p, int arith, int m, const pbt::SolveArgs
         !encode_lines(&maps.w, g.cw, g.nsys, g.nrow, ls, mm, m, &rf) || !rf)
         return false;
     if (arith == kFF)
-        *e = m == 3 ? pbt::launch_transposed_ring<pbt::FF, 3>(g, ls, maps) : pbt::launch_transposed_ring<pbt::FF, 4>(g, ls, maps);
+        *e = m == 3 ? pbt::launch_transposed_ring<pbt::FF, 3>(g, ls, maps, p->redo)
+                    : pbt::launch_transposed_ring<pbt::FF, 4>(g, ls, maps, p->redo);
     else
         switch (m) {
-            case 3: *e = pbt::launch_transposed_ring<pbt::F64, 3>(g, ls, maps); break;
-            case 4: *e = pbt::launch_transposed_ring<pbt::F64, 4>(g, ls, maps); break;
-            case 5: *e = pbt::launch_transposed_ring<pbt::F64, 5>(g, ls, maps); break;
-            default: *e = pbt::launch_transposed_ring<pbt::F64, 6>(g, ls, maps); break;
+            case 3: *e = pbt::launch_transposed_ring<pbt::F64, 3>(g, ls, maps, p->redo); break;
+            case 4: *e = pbt::launch_transposed_ring<pbt::F64, 4>(g, ls, maps, p->redo); break;
+            case 5: *e = pbt::launch_transposed_ring<pbt::F64, 5>(g, ls, maps, p->redo); break;
+            default: *e = pbt::launch_transposed_ring<pbt::F64, 6>(g, ls, maps, p->redo); break;
         }
     return *e != cudaErrorNotSupported;
 }
 
+// M^T lambda = g (in g.d) of a single-segment plan, straight from the stored
+// blocks: by column lanes or through the ring where the forward solve takes
+// them; false: neither, not launched.
+bool transposed_launch(const pbt_plan* p, int arith, int m, const pbt::SolveArgs& g, cudaError_t* e) {
+    bool ring = false;
+    if (p->twisted || thomas_cols(p, arith, m))
+        *e = run_transposed_cols(p, arith, m, g, p->twisted);
+    else if (!(ring = transposed_ring(p, arith, m, g, e))) {
+        if (!p->guarded) return false;
+        *e = run_transposed_cols(p, arith, m, g, 0);
+    }
+    if (p->guarded && *e == cudaSuccess) *e = run_redo_cols(p, arith, m, g, 1, ring);
+    return true;
+}
+
 cudaError_t thomas_launch(const pbt_plan* p, int arith, int m, const pbt::SolveArgs& g) {
     const pbt::LineStrides plain{g.nsys, 1, 0, g.nsys, (long long)g.nsys * g.nrow};
-    if (p->twisted) return run_twist_cols(arith, m, g);
-    if (thomas_cols(p, arith, m)) return run_thomas_cols(arith, m, g, plain);
     cudaError_t e;
+    if (p->guarded) {  // by columns too where past cols_pay's line the ring is not to be had
+        bool ring = false;
+        if (p->twisted)
+            e = run_twist_cols(p, arith, m, g);
+        else if (thomas_cols(p, arith, m) || !(ring = ring_launch(p, arith, m, g, plain, &e)))
+            e = run_thomas_cols(p, arith, m, g, plain);
+        return e == cudaSuccess ? run_redo_cols(p, arith, m, g, 0, ring) : e;
+    }
+    if (thomas_cols(p, arith, m)) return run_thomas_cols(p, arith, m, g, plain);
     if (ring_launch(p, arith, m, g, plain, &e)) return e;
     pbt::ThomasMaps maps;
     return thomas_stages(p, arith, m, g, &maps) ? run_thomas_staged(arith, m, g, maps) : run_thomas(arith, m, g);
@@ -579,11 +606,12 @@ bool one_segment_pays(const pbt_plan_desc& d, int sms) {
 }
 
 // Plans whose method is the library's choice: nseg > 1, non-cyclic, FP64 or
-// float-float, the factors not the caller's (in place), the reference method
-// not asked for.
+// float-float, the factors not the caller's (in place), neither the reference
+// method nor a way to load asked for.
 bool method_free(const pbt_plan_desc& d) {
     return d.nseg > 1 && d.precision != PBT_PREC_FP32_REFINE &&
-           !(d.flags & (PBT_FLAG_CYCLIC | PBT_FLAG_INPLACE | PBT_FLAG_REFERENCE_METHOD));
+           !(d.flags & (PBT_FLAG_CYCLIC | PBT_FLAG_INPLACE | PBT_FLAG_REFERENCE_METHOD | PBT_FLAG_DIRECT_LOADS |
+                        PBT_FLAG_STAGED_LOADS));
 }
 // Whether such a plan solves its lines from both ends at once (the twisted form
 // of pbt_cols.cuh: half the chain of one segment at the same arithmetic, against
@@ -597,7 +625,7 @@ bool method_free(const pbt_plan_desc& d) {
 // -> 1961, 8000 4403 / 4549 -> 5872 (past residency); m = 8, 800 x 512 in 16
 // 5035 / 6325 -> 3501.
 bool twisted_pays(const pbt_plan_desc& d, int sms) {
-    if (!method_free(d) || (d.flags & (PBT_FLAG_DIRECT_LOADS | PBT_FLAG_STAGED_LOADS)) || d.threads_per_block) return false;
+    if (!method_free(d) || d.threads_per_block) return false;
     const int arith = arith_of(d.precision), per = 32 / (d.m + 1);
     const long long n = sms > 0 ? sms : 152, warps = 2LL * ((d.nsys + per - 1) / per);
     if (!cols_pay(arith, d.m, d.nsys, false, sms) || warps > n * (d.m <= 3 ? 48 : d.m <= 6 ? 16 : 12)) return false;
@@ -700,6 +728,8 @@ void free_plan(pbt_plan* p) {
     cudaFree(p->rd);
     cudaFree(p->re);
     cudaFree(p->status);
+    cudaFree(p->redo);
+    p->redo = nullptr;
     p->aw = p->cw = p->ra = p->rc = p->rd = p->re = nullptr;
     p->status = nullptr;
 }
@@ -913,21 +943,8 @@ int solve_core(pbt_plan* p, double* a, double* b, double* c, double* d, int m, i
 
     // A profiled solve reports the phases of the segments that the caller asked
     // for: where the library's own measurements would solve a batch that does
-    // not fill the GPU without them, it runs the two-stage method (whose
-    // workspace the first such call allocates).
-    const bool phases = timed && p->thomas && !p->lines;
-    if (phases && !p->ra) {
-        const size_t mm = (size_t)m * m, rows = (size_t)nsys * nrow, rrows = (size_t)nsys * 2 * ds.nseg, had = p->bytes;
-        if ((rc = alloc(p, &p->aw, mm * rows)) || (rc = alloc(p, &p->rc, mm * rrows)) ||
-            (rc = alloc(p, &p->rd, (size_t)m * rrows)) || (rc = alloc(p, &p->ra, mm * rrows))) {
-            cudaFree(p->aw);
-            cudaFree(p->rc);
-            cudaFree(p->rd);
-            p->aw = p->rc = p->rd = nullptr;
-            p->bytes = had;
-            return rc;
-        }
-    }
+    // not fill the GPU without them, it runs the two-stage method.
+    const bool phases = timed && p->guarded;
     cudaError_t e;
     if ((e = mark(0)) != cudaSuccess) return cuda_fail(e, "cudaEventRecord");
     if (ds.precision == PBT_PREC_FP32_REFINE) {
@@ -1042,24 +1059,26 @@ int pbt_plan_create_ex(pbt_plan** out, const pbt_plan_desc* desc) {
     const bool one_seg = full || p->twisted || (method_free(d) && one_segment_pays(d, p->sms));
     p->thomas = one_seg && !cyclic && !(d.flags & PBT_FLAG_REFERENCE_METHOD);
     p->lines = p->thomas && full;
+    p->guarded = p->thomas && !full;
     p->cyclic_thomas = one_seg && cyclic;
     const size_t mm = (size_t)d.m * d.m;
     const size_t rows = (size_t)d.nsys * d.nrow;
     const size_t rrows = (size_t)d.nsys * 2 * d.nseg;
     if (!inplace) {
         if ((rc = alloc(p, &p->cw, mm * rows))) goto fail_out;
-        // aw: A' for the two-stage method; for a single-segment refined plan,
-        // the FP32 factors its first pass keeps: per row and warp of 32
+        // aw: A' for the two-stage method (and before it a guarded plan's d);
+        // for a single-segment refined plan, the FP32 factors its first pass keeps: per row and warp of 32
         // systems, m*m + 1 runs of 32 floats.
         const bool keep_lu = p->thomas && d.precision == PBT_PREC_FP32_REFINE && d.m <= pbt::kStagedMaxBlock;
         const size_t lu_doubles = (size_t)d.nrow * ((d.nsys + 31) / 32) * 16 * (mm + 1);
-        if (!p->thomas && !p->cyclic_thomas && (rc = alloc(p, &p->aw, mm * rows))) goto fail_out;
+        const bool two_stage = (!p->thomas && !p->cyclic_thomas) || p->guarded;
+        if (two_stage && (rc = alloc(p, &p->aw, mm * rows))) goto fail_out;
         if (keep_lu && (rc = alloc(p, &p->aw, lu_doubles))) goto fail_out;
     }
     if (p->cyclic_thomas) {
         // The fill-in column of every row (also with PBT_FLAG_INPLACE).
         if ((rc = alloc(p, &p->re, mm * rows))) goto fail_out;
-    } else if (!p->thomas) {
+    } else if (!p->thomas || p->guarded) {
         if ((rc = alloc(p, &p->ra, mm * rrows))) goto fail_out;
         if ((rc = alloc(p, &p->rc, mm * rrows))) goto fail_out;
         if ((rc = alloc(p, &p->rd, (size_t)d.m * rrows))) goto fail_out;
@@ -1093,6 +1112,15 @@ int pbt_plan_create_ex(pbt_plan** out, const pbt_plan_desc* desc) {
             rc = cuda_fail(e, "plan_create: refinement statistic");
             goto fail_out;
         }
+    }
+    if (p->guarded) {
+        cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&p->redo), (size_t)d.nsys);
+        if (e == cudaSuccess) e = cudaMemset(p->redo, 0, (size_t)d.nsys);
+        if (e != cudaSuccess) {
+            rc = cuda_fail(e, "plan_create: flags of the guarded solve");
+            goto fail_out;
+        }
+        p->bytes += (size_t)d.nsys;
     }
     {
         cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&p->status), sizeof(unsigned long long));
@@ -1217,7 +1245,7 @@ int pbt_solve_noncyclic_lines(pbt_plan* p, double* a, double* b, double* c, doub
     const pbt::SolveArgs g = make_args(p, a, b, c, d, s, ds.nsys);
     cudaError_t e;
     if (thomas_cols(p, arith, ds.m))
-        e = run_thomas_cols(arith, ds.m, g, ls);
+        e = run_thomas_cols(p, arith, ds.m, g, ls);
     else if (!ring_launch(p, arith, ds.m, g, ls, &e))
         e = run_thomas_lines(arith, ds.m, g, ls);
     if (e != cudaSuccess) return cuda_fail(e, "block Thomas launch (strided lines)");
@@ -1311,24 +1339,18 @@ int pbt_adjoint_noncyclic(pbt_plan* p, const double* a, const double* b, const d
         if (e != cudaSuccess) return cuda_fail(e, "adjoint launch");
         return PBT_OK;
     }
-    // Plans of nseg > 1: materialise M^T and solve it with the plan's own
-    // forward method.
+    // Plans that run the two-stage method: materialise M^T and solve it so.
     if (!p->at) {
         const size_t n = (size_t)ds.m * ds.m * ds.nsys * ds.nrow;
         if ((rc = alloc(p, &p->at, n)) || (rc = alloc(p, &p->bt, n)) || (rc = alloc(p, &p->ct, n))) return rc;
     }
     if ((e = run_transpose_blocks(m, g0, p->at, p->bt, p->ct)) != cudaSuccess)
         return cuda_fail(e, "adjoint: transpose launch");
-    if (p->thomas) {
-        e = thomas_launch(p, arith, m, make_args(p, p->at, p->bt, p->ct, g, s, ds.nsys));
-        if (e != cudaSuccess) return cuda_fail(e, "adjoint: transposed solve launch");
-    } else {
-        pbt::SolveArgs gs = make_args(p, p->at, p->bt, p->ct, g, s, ds.nsys * ds.nseg);
-        if ((e = local_launch(p, arith, m, gs)) != cudaSuccess ||
-            (e = reduced_launch(p, arith, m, make_args(p, p->at, p->bt, p->ct, g, s, ds.nsys))) != cudaSuccess ||
-            (e = run_update(arith, m, gs)) != cudaSuccess)
-            return cuda_fail(e, "adjoint: transposed solve launch");
-    }
+    const pbt::SolveArgs gs = make_args(p, p->at, p->bt, p->ct, g, s, ds.nsys * ds.nseg);
+    if ((e = local_launch(p, arith, m, gs)) != cudaSuccess ||
+        (e = reduced_launch(p, arith, m, make_args(p, p->at, p->bt, p->ct, g, s, ds.nsys))) != cudaSuccess ||
+        (e = run_update(arith, m, gs)) != cudaSuccess)
+        return cuda_fail(e, "adjoint: transposed solve launch");
     if ((e = run_gradients(m, g0, adj)) != cudaSuccess) return cuda_fail(e, "adjoint: gradient launch");
     return PBT_OK;
 }

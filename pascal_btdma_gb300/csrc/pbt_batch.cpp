@@ -23,6 +23,7 @@ struct pbt_batch {
     int rows3[PBT_MAX_BLOCK + 1] = {};  // rows of the longest segment of items3
     std::vector<int> order;
     int off_cols = 0, cnt_cols = 0;  // items1 of k_batch_cols (0: not used)
+    bool cols_redo = false;          // lines of several segments among them
     std::vector<long long> user_mat_off, user_vec_off;
     long long user_mat = 0, user_vec = 0, packed_mat = 0, packed_vec = 0, red_mat = 0, red_vec = 0;
     // device
@@ -37,6 +38,7 @@ struct pbt_batch {
     int pack_chunks = 0;
     int* state = nullptr;  // error (always 0), pad, head1[m] (kHeads), seg_done[ntiles]
     unsigned long long* status = nullptr;
+    unsigned char* redo = nullptr;  // with cols_redo: a flag a lane of every tile, clear between solves
     double *aw = nullptr, *cw = nullptr, *ra = nullptr, *rc = nullptr, *rd = nullptr;
     cudaStream_t last_stream = nullptr;
     unsigned magic = 0x50425442u;  // "PBTB"
@@ -110,6 +112,7 @@ void free_batch(pbt_batch* b) {
     cudaFree(b->chunk_start);
     cudaFree(b->state);
     cudaFree(b->status);
+    cudaFree(b->redo);
     cudaFree(b->aw);
     cudaFree(b->cw);
     cudaFree(b->ra);
@@ -232,7 +235,8 @@ int pbt_batch_create(pbt_batch** out, int nsys, const int* m, const int* nrow, i
     for (auto& t : tiles) {
         t.red_mat_off = red_m;
         t.red_vec_off = red_v;
-        if (t.nseg > 1 && !by_cols(t)) {
+        if (t.nseg > 1) {
+            b->cols_redo |= by_cols(t);
             red_m += 32LL * 2 * t.nseg * t.m * t.m;
             red_v += 32LL * 2 * t.nseg * t.m;
         }
@@ -333,6 +337,10 @@ int pbt_batch_create(pbt_batch** out, int nsys, const int* m, const int* nrow, i
         if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&b->status), sizeof(unsigned long long));
         if (e == cudaSuccess) e = cudaMemset(b->status, 0, sizeof(unsigned long long));
         if (e == cudaSuccess) e = cudaMemset(b->state, 0, sizeof(int) * state_ints(b->ntiles));
+        if (e == cudaSuccess && b->cols_redo) {
+            e = cudaMalloc(reinterpret_cast<void**>(&b->redo), (size_t)b->ntiles * 32);
+            if (e == cudaSuccess) e = cudaMemset(b->redo, 0, (size_t)b->ntiles * 32);
+        }
         if (e != cudaSuccess) {
             rc = bcuda(e, "batch_create: queue state");
             goto fail_out;
@@ -431,6 +439,7 @@ int pbt_batch_solve(pbt_batch* b, const double* pa, const double* pb, const doub
     ba.tiles = b->tiles;
     ba.lane_rows = b->lane_rows;
     ba.status = b->status;
+    ba.redo = b->redo;
     ba.seg_done = b->state + 2 + kHeads;
     b->last_grid = 0;
     if (b->cnt_cols > 0) {
@@ -440,6 +449,8 @@ int pbt_batch_solve(pbt_batch* b, const double* pa, const double* pb, const doub
         ba.n3 = ba.rows3 = 0;
         ba.head1 = nullptr;
         if ((e = pbt::launch_batch_cols(ba, b->precision == PBT_PREC_FF, s)) != cudaSuccess)
+            return bcuda(e, "batch_solve: launch");
+        if (b->cols_redo && (e = pbt::launch_batch_redo(ba, b->precision == PBT_PREC_FF, s)) != cudaSuccess)
             return bcuda(e, "batch_solve: launch");
         b->last_grid = b->cnt_cols / pbt::batch_cols_pairs(b->precision == PBT_PREC_FF);
     }

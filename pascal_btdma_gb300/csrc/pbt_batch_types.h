@@ -36,6 +36,7 @@ struct BatchArgs {
     int* head1;            // queue head, zeroed before every solve
     int* seg_done;         // per tile: segments done (zeroed before every solve)
     unsigned long long* status;  // zero pivots, range flag
+    unsigned char* redo = nullptr;  // [tile*32 + lane]: lines that k_batch_cols left to k_batch_redo
 };
 
 // Packing between the caller's per-system layout and the tiled layout.
@@ -58,6 +59,9 @@ constexpr int kBatchColsMaxBlock = 6;
 constexpr int kBatchColsMaxPairs = 4;
 constexpr int batch_cols_pairs(bool ff) { return ff ? kBatchColsMaxPairs : 1; }
 cudaError_t launch_batch_cols(const BatchArgs& ba, int ff, cudaStream_t s);
+// Lines of several segments whose elimination from both ends met a zero pivot or
+// grew, in their segments; after launch_batch_cols.
+cudaError_t launch_batch_redo(const BatchArgs& ba, int ff, cudaStream_t s);
 
 // The launches of block size M (pbt_batch.cuh; instantiated with the other
 // kernels of (Num, M) in pbt_inst.cu).

@@ -206,18 +206,34 @@ __host__ __device__ constexpr int cols_ahead() {
 // I, everything raw; A, C', d in RA, RC, RD); Transposed: A, B and C hold the
 // transposed blocks (column j of a block is row j of what is stored).
 //
+// Guard: for lines that the plan cuts into segments, whose two-stage method
+// needs other blocks to be regular than an elimination from the ends does (the
+// last block, singular in a line closed by a constraint, is one that it never
+// inverts).  The forward sweep leaves y in Y instead of D and follows the size
+// of C' (kGrowthExp).  A line that met a zero pivot or grew past it keeps d, its
+// flag *redo is set, and k_redo_cols solves it in its segments; otherwise D takes
+// x.  Unguarded -> guarded, us, where nothing is redone: FP64 m = 3, 1024 x 128
+// 151.5 -> 153.6 (2 of it k_redo_cols' launch), float-float m = 3, 12347 x 301
+// 642 -> 663, FP64 m = 8, 4096 x 1024 24886 -> 25012; where every line is:
+// FP64 m = 5, 1000 x 128 in 4 432 -> 986 (the two-stage method alone, one thread a
+// segment, 1569).
+//
 // Twisted: the line is eliminated from both ends at once, by two warps of a
 // CTA (the pair's `side` 0 from the first row on, 1 from the last row on with A
 // and C in each other's place and a negative row stride), N rows each.  Where
 // they meet, x = y - P x' on either side (P the last C', x', P' and y' the
 // other side's), so x = (I - P P')^{-1} (y - P y'); then both substitute back
 // outwards.  Half the chain of block Thomas at the same arithmetic.  `sh`: the
-// pair's exchange, 2 x 32 lanes x M values.
-template <class Num, int M, bool Reduced, bool Transposed = false, bool Twisted = false>
+// pair's exchange (kTwistShared).  Always guarded.
+template <int M>
+constexpr int kTwistShared = 2 * 32 * M + 32;  // doubles: 32 lanes x M values, then a flag a lane, of either side
+template <class Num, int M, bool Reduced, bool Transposed = false, bool Twisted = false, bool Guard = Twisted>
 __device__ __forceinline__ void thomas_cols_body(const double* A, const double* B, const double* C, double* D,
                                                  double* CW, size_t plane, ptrdiff_t rs, int N, bool raw,
-                                                 unsigned long long* status, const ColLane& cl, int side = 0,
-                                                 double* sh = nullptr, int bar = 1) {
+                                                 unsigned long long* status, const ColLane& cl, double* Y = nullptr,
+                                                 unsigned char* redo = nullptr, int side = 0, double* sh = nullptr,
+                                                 int bar = 1) {
+    static_assert(Guard || !Twisted, "elimination from both ends is guarded");
     using T = typename Num::T;
     using Acc = typename Num::Acc;
     const bool rhs = cl.j == M;
@@ -228,8 +244,10 @@ __device__ __forceinline__ void thomas_cols_body(const double* A, const double* 
     const double* const pa = A + in;
     const double* const pb = rhs ? D : (Reduced ? A : B + in);
     const double* const pc = C + in;
-    double* const pw = rhs ? D : CW + col;
+    double* const yw = Guard ? Y : D;
+    double* const pw = rhs ? yw : CW + col;
     unsigned bad = 0, amax = 0;
+    [[maybe_unused]] float size = 0.f;  // of C'
     double va[M], vb[M], vc[M];
     T cp[M];
     // Raw inputs of row 0 (A_0 is not read).
@@ -267,8 +285,11 @@ __device__ __forceinline__ void thomas_cols_body(const double* A, const double* 
         for (int i = 0; i < M; ++i) x[0][i] = Num::asel(rhs, r[i], x[0][i]);
         col_gesv<Num, M, 1>(r, x, cl, bad);
 #pragma unroll
-        for (int i = 0; i < M; ++i) cp[i] = Num::fin(x[0][i]);
-        if (cl.live && (Twisted ? !last : rhs || !last)) {
+        for (int i = 0; i < M; ++i) {
+            cp[i] = Num::fin(x[0][i]);
+            if constexpr (Guard) size = max_nan(size, Num::size(cp[i]));
+        }
+        if (cl.live && (Guard ? !last : rhs || !last)) {
 #pragma unroll
             for (int i = 0; i < M; ++i) {
                 double* const p = pw + o + (size_t)i * plane;
@@ -280,31 +301,42 @@ __device__ __forceinline__ void thomas_cols_body(const double* A, const double* 
             }
         }
     }
-    if constexpr (Twisted) {
-        // This side's P and y (cp) against the other's, lane by lane.
-        double* const mine = sh + (side * 32 + (threadIdx.x & 31)) * M;
-        const double* const other = sh + ((side ^ 1) * 32 + (threadIdx.x & 31)) * M;
+    bool keep = cl.live;
+    if constexpr (Guard) {
+        unsigned again = bad | (unsigned)(!rhs && Num::grown(size)), none = 0;
+        col_merge<M>(again, none, cl);
+        if constexpr (Twisted) {
+            // This side's P and y (cp) and its outcome against the other's, lane by lane.
+            const int lane = threadIdx.x & 31;
+            double* const mine = sh + (side * 32 + lane) * M;
+            const double* const other = sh + ((side ^ 1) * 32 + lane) * M;
+            unsigned* const flags = reinterpret_cast<unsigned*>(sh + 2 * 32 * M) + lane;
 #pragma unroll
-        for (int i = 0; i < M; ++i) Num::sts(mine + i, cp[i]);
-        pair_barrier(bar);
-        T oc[M];
-        Acc r[M], x[1][M];
+            for (int i = 0; i < M; ++i) Num::sts(mine + i, cp[i]);
+            flags[side * 32] = again;
+            pair_barrier(bar);
+            again |= flags[(side ^ 1) * 32];
+            T oc[M];
+            Acc r[M], x[1][M];
 #pragma unroll
-        for (int i = 0; i < M; ++i) {
-            oc[i] = Num::lds(other + i);
-            r[i] = rhs ? Num::acc(cp[i]) : Num::acc(i == cl.j ? Num::one() : Num::zero());
+            for (int i = 0; i < M; ++i) {
+                oc[i] = Num::lds(other + i);
+                r[i] = rhs ? Num::acc(cp[i]) : Num::acc(i == cl.j ? Num::one() : Num::zero());
+            }
+            col_product<Num, M>(r, cp, oc, cl.base);
+#pragma unroll
+            for (int i = 0; i < M; ++i) x[0][i] = Num::asel(rhs, r[i], Num::acc0());
+            col_gesv<Num, M, 1>(r, x, cl, bad);
+#pragma unroll
+            for (int i = 0; i < M; ++i) cp[i] = Num::fin(x[0][i]);
         }
-        col_product<Num, M>(r, cp, oc, cl.base);
+        keep = cl.live && again == 0;
+        if (keep && rhs) {
+            double* const p = D + (N - 1) * rs;
 #pragma unroll
-        for (int i = 0; i < M; ++i) x[0][i] = Num::asel(rhs, r[i], Num::acc0());
-        col_gesv<Num, M, 1>(r, x, cl, bad);
-        const ptrdiff_t o = (N - 1) * rs;
-#pragma unroll
-        for (int i = 0; i < M; ++i) {
-            cp[i] = Num::fin(x[0][i]);
-            if (cl.live && rhs) {
+            for (int i = 0; i < M; ++i) {
                 amax = max(amax, Num::mag(cp[i]));
-                Num::out(pw + o + (size_t)i * plane, cp[i]);
+                Num::out(p + (size_t)i * plane, cp[i]);
             }
         }
     }
@@ -316,10 +348,12 @@ __device__ __forceinline__ void thomas_cols_body(const double* A, const double* 
     for (int k = 0; k < M; ++k) xn[k] = col_bcast(cp[k], cl.base + M);
     const size_t mine = (size_t)(rhs ? 0 : cl.j) * plane;
     const double* const pr = CW + mine;  // row j of C'
-    double* const py = D + mine;
+    const double* const py = yw + mine;
+    double* const px = D + mine;
+    const bool back = keep && !rhs;
     double bc[kAhead][M], by[kAhead];
     auto fetch = [&](int slot, int q) {
-        const bool on = mat && q >= 0;
+        const bool on = back && q >= 0;
         const ptrdiff_t o = (q >= 0 ? q : 0) * rs;
         by[slot] = on ? py[o] : 0.0;
 #pragma unroll
@@ -344,12 +378,12 @@ __device__ __forceinline__ void thomas_cols_body(const double* A, const double* 
                 }
                 const T xq = Num::fin(t);
                 fetch(s, q - kAhead);
-                if (mat) {
+                if (back) {
                     amax = max(amax, Num::mag(xq));
                     if (Reduced)
-                        Num::sts(py + o, xq);
+                        Num::sts(px + o, xq);
                     else
-                        Num::out(py + o, xq);
+                        Num::out(px + o, xq);
                 }
 #pragma unroll
                 for (int k = 0; k < M; ++k) xn[k] = col_bcast(xq, cl.base + k);
@@ -366,10 +400,17 @@ __device__ __forceinline__ void thomas_cols_body(const double* A, const double* 
             u[1] = amax;
         }
         pair_barrier(bar);
-        if (side == 0 && cl.live && cl.j == 0)
-            report_status(status, bad | u[0] | range_bits<Num>(max(amax, u[1]), true));
+        if (side == 0 && cl.live && cl.j == 0) {
+            if (keep)
+                report_status(status, bad | u[0] | range_bits<Num>(max(amax, u[1]), true));
+            else
+                *redo = 1;
+        }
     } else {
-        col_report<Num, M>(status, bad, amax, true, cl);
+        if (Guard && cl.live && !keep && cl.j == 0) *redo = 1;
+        ColLane out = cl;
+        out.live = keep;
+        col_report<Num, M>(status, bad, amax, true, out);
     }
 }
 
@@ -383,13 +424,15 @@ template <int M>
 __host__ __device__ constexpr int cols_warps() {
     return 4 * cols_min_ctas<M>(false);
 }
-template <class Num, int M>
-__global__ void __launch_bounds__(32 * cols_warps<M>(), 1) k_thomas_cols(const SolveArgs g, const LineStrides ls) {
+template <class Num, int M, bool Guard>
+__global__ void __launch_bounds__(32 * cols_warps<M>(), 1) k_thomas_cols(const SolveArgs g, const LineStrides ls,
+                                                                       unsigned char* redo) {
     const ColLane cl = col_lane<M>(g.nsys, grid_warp());
     const long long s = cl.live ? cl.sys : 0;
     const size_t o = (size_t)(s % ls.lin) * (size_t)ls.in + (size_t)(s / ls.lin) * (size_t)ls.out;
-    thomas_cols_body<Num, M, false>(g.a + o, g.b + o, g.c + o, g.d + o, g.cw + o, (size_t)ls.elem, (size_t)ls.row,
-                                    g.nrow, g.factors_raw != 0, g.status, cl);
+    thomas_cols_body<Num, M, false, false, false, Guard>(g.a + o, g.b + o, g.c + o, g.d + o, g.cw + o, (size_t)ls.elem,
+                                                         (size_t)ls.row, g.nrow, g.factors_raw != 0, g.status, cl,
+                                                         Guard ? g.aw + o : nullptr, Guard ? redo + s : nullptr);
 }
 
 template <class Num, int M>
@@ -403,52 +446,66 @@ __global__ void __launch_bounds__(128, cols_min_ctas<M>(false)) k_reduced_cols(c
 // M^T lambda = g for the adjoint, from the forward blocks as they are stored:
 // At_q = C_{q-1}^T, Bt_q = B_q^T, Ct_q = A_{q+1}^T; lambda in D, the factors in
 // the workspace (raw).
-template <class Num, int M>
-__global__ void __launch_bounds__(32 * cols_warps<M>(), 1) k_transposed_cols(const SolveArgs g) {
+template <class Num, int M, bool Guard>
+__global__ void __launch_bounds__(32 * cols_warps<M>(), 1) k_transposed_cols(const SolveArgs g, unsigned char* redo) {
     const ColLane cl = col_lane<M>(g.nsys, grid_warp());
     const size_t s = cl.live ? (size_t)cl.sys : 0, rs = (size_t)g.nsys;
-    thomas_cols_body<Num, M, false, true>(g.c + s - rs, g.b + s, g.a + s + rs, g.d + s, g.cw + s, rs * g.nrow, rs,
-                                          g.nrow, true, g.status, cl);
+    thomas_cols_body<Num, M, false, true, false, Guard>(g.c + s - rs, g.b + s, g.a + s + rs, g.d + s, g.cw + s,
+                                                        rs * g.nrow, rs, g.nrow, true, g.status, cl,
+                                                        Guard ? g.aw + s : nullptr, Guard ? redo + s : nullptr);
 }
 
 // The twisted solve, one pair of warps a CTA; Transposed: of M^T, as above.
 template <class Num, int M, bool Transposed>
-__global__ void __launch_bounds__(64, 2 * cols_min_ctas<M>(false)) k_twist_cols(const SolveArgs g) {
-    __shared__ double sh[2 * 32 * M];
+__global__ void __launch_bounds__(64, 2 * cols_min_ctas<M>(false)) k_twist_cols(const SolveArgs g, unsigned char* redo) {
+    __shared__ double sh[kTwistShared<M>];
     const ColLane cl = col_lane<M>(g.nsys, blockIdx.x);
     const int side = threadIdx.x >> 5, n0 = g.nrow / 2, n = side ? g.nrow - n0 : n0;
-    const ptrdiff_t rs = g.nsys;
+    const ptrdiff_t rs = g.nsys, s = cl.live ? (ptrdiff_t)cl.sys : 0;
     const size_t plane = (size_t)g.nsys * g.nrow;
-    const ptrdiff_t o = (cl.live ? (ptrdiff_t)cl.sys : 0) + (side ? rs * (g.nrow - 1) : 0);
+    const ptrdiff_t o = s + (side ? rs * (g.nrow - 1) : 0);
     const double* const a = Transposed ? g.c - rs : g.a;  // row q of the lower blocks at a + o + q * rs
     const double* const c = Transposed ? g.a + rs : g.c;
     thomas_cols_body<Num, M, false, Transposed, true>((side ? c : a) + o, g.b + o, (side ? a : c) + o, g.d + o,
-                                                      g.cw + o, plane, side ? -rs : rs, n, true, g.status, cl, side, sh);
+                                                      g.cw + o, plane, side ? -rs : rs, n, true, g.status, cl, g.aw + o,
+                                                      redo + s, side, sh);
 }
 
 // Local stage of one segment of one system per group (modi_body, column per
 // lane): lane j < M carries column j of A' and C', lane M d' (in the place of
-// a C' column).
-template <class Num, int M>
-__global__ void __launch_bounds__(128, cols_min_ctas<M>(true)) k_modi_cols(const SolveArgs g) {
+// a C' column).  Pointers at system 0, rows rs apart, 2 * nseg reduced rows rs
+// apart too; segment rows f .. f + n - 1.  Transposed: A_q, B_q, C_q are
+// C_{q-1}^T, B_q^T, A_{q+1}^T of the blocks in C, B, A (zero past the ends).
+template <class Num, int M, bool Transposed>
+__device__ __forceinline__ void modi_cols_body(const double* A, const double* B, const double* C, double* D, double* AW,
+                                               double* CW, double* RA, double* RC, double* RD, size_t rs, int nrow,
+                                               int nseg, int seg, bool raw, unsigned long long* status,
+                                               const ColLane& cl) {
     using T = typename Num::T;
     using Acc = typename Num::Acc;
-    const ColLane cl = col_lane<M>(g.nsys, grid_warp());
-    const bool rhs = cl.j == M, mat = cl.live && !rhs, raw = g.factors_raw != 0;
-    const int seg = blockIdx.y;
+    const bool rhs = cl.j == M, mat = cl.live && !rhs;
     int f, l;
-    seg_rows(g.nrow, g.nseg, seg, f, l);
+    seg_rows(nrow, nseg, seg, f, l);
     const int n = l - f + 1;
-    const size_t rs = (size_t)g.nsys, plane = rs * g.nrow, s = cl.live ? (size_t)cl.sys : 0;
+    const size_t plane = rs * nrow, s = cl.live ? (size_t)cl.sys : 0;
     const size_t fo = (size_t)f * rs + s, col = (size_t)(rhs ? 0 : cl.j) * M * plane;
-    const double* const pa = g.a + fo + col;
-    const double* const pb = rhs ? g.d + fo : g.b + fo + col;
-    const double* const pc = g.c + fo + col;
-    double* const qa = g.aw + fo + col;
-    double* const qc = rhs ? g.d + fo : g.cw + fo + col;
-    const size_t rplane = rs * 2 * g.nseg, rcol = (size_t)(rhs ? 0 : cl.j) * M * rplane;
-    double* const ra = g.ra + s + rcol;
-    double* const rc = rhs ? g.rd + s : g.rc + s + rcol;
+    const size_t in = Transposed ? (size_t)(rhs ? 0 : cl.j) * plane : col;  // this lane's column of an input block
+    const size_t es = Transposed ? M * plane : plane, eb = Transposed && !rhs ? es : plane;
+    const double* const pa = (Transposed ? C - rs : A) + fo + in;
+    const double* const pb = rhs ? D + fo : B + fo + in;
+    const double* const pc = (Transposed ? A + rs : C) + fo + in;
+    double* const qa = AW + fo + col;
+    double* const qc = rhs ? D + fo : CW + fo + col;
+    const size_t rplane = rs * 2 * nseg, rcol = (size_t)(rhs ? 0 : cl.j) * M * rplane;
+    double* const ra = RA + s + rcol;
+    double* const rc = rhs ? RD + s : RC + s + rcol;
+    const bool no_a = Transposed && f == 0;  // the line's first row has no A^T, its last no C^T
+    auto load = [&](double (&va)[M], double (&vb)[M], double (&vc)[M], int q) {
+        const size_t o = (size_t)q * rs;
+        col_load<M>(va, pa + o, es, mat && !(no_a && q == 0));
+        col_load<M>(vb, pb + o, eb, cl.live);
+        col_load<M>(vc, pc + o, es, mat && !(Transposed && f + q == nrow - 1));
+    };
     unsigned bad = 0;
     // This lane's column of row q into the factor arrays, and into the
     // reduced row rr (rr < 0: none).
@@ -472,9 +529,7 @@ __global__ void __launch_bounds__(128, cols_min_ctas<M>(true)) k_modi_cols(const
     T ap[M], cp[M];
     {
         double va[M], vb[M], vc[M];
-        col_load<M>(va, pa, plane, mat);
-        col_load<M>(vb, pb, plane, cl.live);
-        col_load<M>(vc, pc, plane, mat);
+        load(va, vb, vc, 0);
         for (int q = 0; q < n; ++q) {
             T a[M];
             Acc r[M], x[2][M];
@@ -485,12 +540,7 @@ __global__ void __launch_bounds__(128, cols_min_ctas<M>(true)) k_modi_cols(const
                 x[0][i] = (q < 2) ? Num::acc(a[i]) : Num::acc0();
                 x[1][i] = Num::acc(Num::in_value(vc[i], false));
             }
-            if (q + 1 < n) {
-                const size_t p = (size_t)(q + 1) * rs;
-                col_load<M>(va, pa + p, plane, mat);
-                col_load<M>(vb, pb + p, plane, cl.live);
-                col_load<M>(vc, pc + p, plane, mat);
-            }
+            if (q + 1 < n) load(va, vb, vc, q + 1);
             if (q >= 2) col_product2<Num, M>(r, x[0], a, cp, ap, cl.base);
 #pragma unroll
             for (int i = 0; i < M; ++i) x[1][i] = Num::asel(rhs, r[i], x[1][i]);
@@ -546,7 +596,71 @@ __global__ void __launch_bounds__(128, cols_min_ctas<M>(true)) k_modi_cols(const
             store(q, ap, cp, q == 0 ? 2 * seg : -1);
         }
     }
-    col_report<Num, M>(g.status, bad, 0u, false, cl);
+    col_report<Num, M>(status, bad, 0u, false, cl);
+}
+template <class Num, int M>
+__global__ void __launch_bounds__(128, cols_min_ctas<M>(true)) k_modi_cols(const SolveArgs g) {
+    modi_cols_body<Num, M, false>(g.a, g.b, g.c, g.d, g.aw, g.cw, g.ra, g.rc, g.rd, (size_t)g.nsys, g.nrow, g.nseg,
+                                  blockIdx.y, g.factors_raw != 0, g.status, col_lane<M>(g.nsys, grid_warp()));
+}
+
+// The two-stage method for the flagged lines of one group (the arithmetic and
+// the outcome that a plan in segments has): a CTA's warps take segments, the
+// first one the reduced systems, all threads pieces of the update.  Pointers at
+// system 0 of `nsys`, rows rs apart; with `saved` d is in AW's first planes, else
+// still in D; flags are cleared.  Returns at once where no line of the group is
+// flagged.
+template <class Num, int M, bool Transposed>
+__device__ __forceinline__ void redo_cols_group(const double* A, const double* B, const double* C, double* D, double* AW,
+                                                double* CW, double* RA, double* RC, double* RD, size_t rs, int nsys,
+                                                int nrow, int nseg, long long group, unsigned char* redo, bool saved,
+                                                unsigned long long* status) {
+    constexpr int S = cols_systems<M>();
+    ColLane cl = col_lane<M>(nsys, group);
+    cl.live = cl.live && redo[cl.sys] != 0;
+    if (!__syncthreads_or(cl.live)) return;
+    const int per = blockDim.x / S, part = threadIdx.x / S;  // rows or pieces at a time
+    const long long sys = group * S + threadIdx.x % S;
+    const bool mine = part < per && sys < nsys && redo[sys] != 0;
+    if (saved && mine) {
+        for (long long r = part; r < (long long)M * nrow; r += per)
+            D[(size_t)r * rs + (size_t)sys] = AW[(size_t)r * rs + (size_t)sys];
+    }
+    __syncthreads();
+    const int warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    for (int seg = warp; seg < nseg; seg += warps)
+        modi_cols_body<Num, M, Transposed>(A, B, C, D, AW, CW, RA, RC, RD, rs, nrow, nseg, seg, true, status, cl);
+    __syncthreads();
+    if (warp == 0) {
+        const size_t s = cl.live ? (size_t)cl.sys : 0;
+        thomas_cols_body<Num, M, true>(RA + s, nullptr, RC + s, RD + s, RC + s, rs * 2 * nseg, (ptrdiff_t)rs, 2 * nseg,
+                                       true, status, cl);
+    }
+    __syncthreads();
+    unsigned amax = 0;
+    if (mine) {
+        const int pieces = ((nrow + nseg - 1) / nseg + kUpdateRows - 1) / kUpdateRows;
+        for (long long u = part; u < (long long)nseg * pieces; u += per) {
+            const int seg = (int)(u / pieces), q0 = (int)(u % pieces) * kUpdateRows;
+            int f, l;
+            seg_rows(nrow, nseg, seg, f, l);
+            const int n = l - f + 1, q1 = min(n, q0 + kUpdateRows);
+            const size_t o = (size_t)f * rs + (size_t)sys;
+            if (q0 < n)
+                update_rows<Num, M, true>(AW + o, CW + o, D + o, rs * nrow, rs, n, q0, q1, RD + sys, rs * 2 * nseg, rs,
+                                          seg, amax);
+        }
+    }
+    report_status(status, range_bits<Num>(amax, false));
+    __syncthreads();
+    if (mine && part == 0) redo[sys] = 0;
+}
+// One CTA a group: where nothing is flagged, 3.5 us a launch of 1544 CTAs.
+template <class Num, int M, bool Transposed>
+__global__ void __launch_bounds__(128, cols_min_ctas<M>(true)) k_redo_cols(const SolveArgs g, unsigned char* redo,
+                                                                             bool saved) {
+    redo_cols_group<Num, M, Transposed>(g.a, g.b, g.c, g.d, g.aw, g.cw, g.ra, g.rc, g.rd, (size_t)g.nsys, g.nsys,
+                                        g.nrow, g.nseg, blockIdx.x, redo, saved, g.status);
 }
 
 // CTA of the local stage and the reduced solve: one warp while there are fewer
@@ -583,24 +697,29 @@ inline unsigned cols_grid(int nsys, int tpb) {
 }
 
 template <class Num, int M>
-cudaError_t launch_thomas_cols(const SolveArgs& g, const LineStrides& ls) {
+cudaError_t launch_thomas_cols(const SolveArgs& g, const LineStrides& ls, unsigned char* redo) {
     const int tpb = cols_threads_even<Num, M>(g);
-    k_thomas_cols<Num, M><<<cols_grid<M>(g.nsys, tpb), tpb, 0, g.stream>>>(g, ls);
+    const auto kernel = redo ? k_thomas_cols<Num, M, true> : k_thomas_cols<Num, M, false>;
+    kernel<<<cols_grid<M>(g.nsys, tpb), tpb, 0, g.stream>>>(g, ls, redo);
     return cudaGetLastError();
 }
 template <class Num, int M>
-cudaError_t launch_twist_cols(const SolveArgs& g) {
-    k_twist_cols<Num, M, false><<<cols_grid<M>(g.nsys, 32), 64, 0, g.stream>>>(g);
+cudaError_t launch_twist_cols(const SolveArgs& g, unsigned char* redo) {
+    k_twist_cols<Num, M, false><<<cols_grid<M>(g.nsys, 32), 64, 0, g.stream>>>(g, redo);
     return cudaGetLastError();
 }
 template <class Num, int M>
-cudaError_t launch_transposed_cols(const SolveArgs& g, int twisted) {
-    if (twisted) {
-        k_twist_cols<Num, M, true><<<cols_grid<M>(g.nsys, 32), 64, 0, g.stream>>>(g);
-        return cudaGetLastError();
-    }
-    const int tpb = cols_threads_even<Num, M>(g);
-    k_transposed_cols<Num, M><<<cols_grid<M>(g.nsys, tpb), tpb, 0, g.stream>>>(g);
+cudaError_t launch_transposed_cols(const SolveArgs& g, int twisted, unsigned char* redo) {
+    const int tpb = twisted ? 64 : cols_threads_even<Num, M>(g);
+    const auto kernel = twisted ? k_twist_cols<Num, M, true>
+                                : (redo ? k_transposed_cols<Num, M, true> : k_transposed_cols<Num, M, false>);
+    kernel<<<cols_grid<M>(g.nsys, twisted ? 32 : tpb), tpb, 0, g.stream>>>(g, redo);
+    return cudaGetLastError();
+}
+template <class Num, int M>
+cudaError_t launch_redo_cols(const SolveArgs& g, int transposed, unsigned char* redo, bool saved) {
+    const auto kernel = transposed ? k_redo_cols<Num, M, true> : k_redo_cols<Num, M, false>;
+    kernel<<<cols_grid<M>(g.nsys, 32), 128, 0, g.stream>>>(g, redo, saved);
     return cudaGetLastError();
 }
 template <class Num, int M>

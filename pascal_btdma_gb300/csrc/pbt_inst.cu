@@ -37,15 +37,18 @@ template cudaError_t launch_update<PBT_NUM, PBT_M>(const SolveArgs&);
 template cudaError_t launch_adjoint<PBT_NUM, PBT_M>(const SolveArgs&, const AdjointArgs&);
 #if defined(PBT_NUM_IS_F64) || defined(PBT_NUM_IS_FF)
 template cudaError_t launch_batch<PBT_NUM, PBT_M>(const BatchArgs&, int, cudaStream_t, int*);
-template cudaError_t launch_thomas_cols<PBT_NUM, PBT_M>(const SolveArgs&, const LineStrides&);
+template cudaError_t launch_thomas_cols<PBT_NUM, PBT_M>(const SolveArgs&, const LineStrides&, unsigned char*);
 template cudaError_t launch_modi_cols<PBT_NUM, PBT_M>(const SolveArgs&);
-template cudaError_t launch_transposed_cols<PBT_NUM, PBT_M>(const SolveArgs&, int);
-template cudaError_t launch_twist_cols<PBT_NUM, PBT_M>(const SolveArgs&);
+template cudaError_t launch_transposed_cols<PBT_NUM, PBT_M>(const SolveArgs&, int, unsigned char*);
+template cudaError_t launch_twist_cols<PBT_NUM, PBT_M>(const SolveArgs&, unsigned char*);
 template cudaError_t launch_reduced_cols<PBT_NUM, PBT_M>(const SolveArgs&);
+template cudaError_t launch_redo_cols<PBT_NUM, PBT_M>(const SolveArgs&, int, unsigned char*, bool);
 #endif
 #ifdef PBT_HAS_RING
-template cudaError_t launch_thomas_ring<PBT_NUM, PBT_M>(const SolveArgs&, const LineStrides&, const ThomasMaps&, int);
-template cudaError_t launch_transposed_ring<PBT_NUM, PBT_M>(const SolveArgs&, const LineStrides&, const ThomasMaps&);
+template cudaError_t launch_thomas_ring<PBT_NUM, PBT_M>(const SolveArgs&, const LineStrides&, const ThomasMaps&, int,
+                                                        unsigned char*);
+template cudaError_t launch_transposed_ring<PBT_NUM, PBT_M>(const SolveArgs&, const LineStrides&, const ThomasMaps&,
+                                                            unsigned char*);
 #endif
 #ifdef PBT_NUM_IS_F64
 template cudaError_t launch_transpose_blocks<PBT_M>(const SolveArgs&, double*, double*, double*);

@@ -79,8 +79,10 @@ cudaError_t launch_lines_layout(const double* src, double* dst, const LineStride
 template <class Num, int M> cudaError_t launch_thomas_staged(const SolveArgs& g, const ThomasMaps& maps);
 // The solve through a CTA-wide ring (pbt_ring.cuh), maps over {lines, rows and
 // outer lines, planes}; cudaErrorNotSupported where its shared memory does not fit.
+// With `redo`: guarded (F64, m >= 4 only).
 template <class Num, int M>
-cudaError_t launch_thomas_ring(const SolveArgs& g, const LineStrides& ls, const ThomasMaps& maps, int row_first);
+cudaError_t launch_thomas_ring(const SolveArgs& g, const LineStrides& ls, const ThomasMaps& maps, int row_first,
+                               unsigned char* redo);
 // Periodic lines in one segment (k_thomas_cyclic): the fill-in column in
 // g.re, nsys * nrow * m * m raw values; nrow >= 3.
 template <class Num, int M> cudaError_t launch_thomas_cyclic(const SolveArgs& g);
@@ -106,17 +108,28 @@ constexpr ColsCost kColsF64 = {{1.0, 1.4, 2.4, 4.2, 5.6, 7.6, 9.3, 12.3, 16.0, 1
 // One lane per block column (pbt_cols.cuh; F64 and FF, m <= kColsMaxBlock),
 // for batches too small for one thread per system: the single-segment solve of
 // lines by strides, the local stage, and the reduced solve.
+// With `redo` (a flag a system, clear) the single-segment solves are guarded: the
+// flag of a line whose elimination met a zero pivot or grew leaves it to
+// launch_redo_cols, its d in g.d (column lanes) or in g.aw's first planes (ring).
 constexpr int kColsMaxBlock = PBT_MAX_BLOCK;
-template <class Num, int M> cudaError_t launch_thomas_cols(const SolveArgs& g, const LineStrides& ls);
+template <class Num, int M>
+cudaError_t launch_thomas_cols(const SolveArgs& g, const LineStrides& ls, unsigned char* redo);
 template <class Num, int M> cudaError_t launch_modi_cols(const SolveArgs& g);
-// The single-segment solve eliminated from both ends (raw factors in g.cw).
-template <class Num, int M> cudaError_t launch_twist_cols(const SolveArgs& g);
+// The single-segment solve eliminated from both ends (raw factors in g.cw),
+// always guarded.
+template <class Num, int M> cudaError_t launch_twist_cols(const SolveArgs& g, unsigned char* redo);
 // M^T x = d for the blocks in a, b, c (x, d in g.d), raw factors in g.cw: one
 // lane a column, and through the CTA's ring (maps.a over C, maps.c over A, with
 // the block's two indices as separate dimensions).
-template <class Num, int M> cudaError_t launch_transposed_cols(const SolveArgs& g, int twisted);
 template <class Num, int M>
-cudaError_t launch_transposed_ring(const SolveArgs& g, const LineStrides& ls, const ThomasMaps& maps);
+cudaError_t launch_transposed_cols(const SolveArgs& g, int twisted, unsigned char* redo);
+template <class Num, int M>
+cudaError_t launch_transposed_ring(const SolveArgs& g, const LineStrides& ls, const ThomasMaps& maps,
+                                   unsigned char* redo);
+// The two-stage method on the plan's segments for the lines that a guarded
+// solve left (of M^T with `transposed`); saved: their d is in g.aw.
+template <class Num, int M>
+cudaError_t launch_redo_cols(const SolveArgs& g, int transposed, unsigned char* redo, bool saved);
 template <class Num, int M> cudaError_t launch_reduced_cols(const SolveArgs& g);
 // Adjoint (pbt_kernels.cuh: k_adjoint, k_transpose_blocks, k_gradients).
 struct AdjointArgs {

@@ -23,6 +23,8 @@
 //   acc(x), mac(acc, x, y) (acc += x*y), msub(acc, x, y) (acc -= x*y), fin(acc)
 //   mul, rcp, neg, zero, one, key (|x| as an ordered integer), sel, is_zero
 //   nonfinite(v), mag(v), kTinyMag: the solution range check (no-ops for F64)
+//   size(v), grown(s): a float that orders |v|, and whether the largest of them
+//                (max_nan) is above 2^kGrowthExp, Inf or NaN (F64 and FF)
 //
 // FP64 <-> FF conversion uses integer bit operations only, so the FF path
 // issues no FP64 instruction except one DADD per FP64 value it writes.
@@ -52,6 +54,19 @@ __device__ __forceinline__ double dsel(unsigned s, double x, double y) {
     asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %3, 0;\n\tselp.f64 %0, %1, %2, p;\n\t}"
         : "=d"(r)
         : "d"(x), "d"(y), "r"(s));
+    return r;
+}
+
+// Solves whose order of elimination the library chose (Guard, pbt_cols.cuh) keep
+// a line's solution only if no element of its C' blocks passed 2^kGrowthExp: what
+// an element loses to a larger one in the sums of the next row, and in the
+// substitution back, is at most that factor.  C' of a block diagonally dominant
+// line stays below 1.
+constexpr unsigned kGrowthExp = 10;
+// The larger value; NaN if either is.
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
     return r;
 }
 
@@ -96,6 +111,10 @@ struct F64 {
     __device__ static __forceinline__ bool nonfinite(T) { return false; }
     __device__ static __forceinline__ unsigned mag(T) { return 0u; }
     static constexpr unsigned kTinyMag = 0u;
+    // The upper word read as a float orders doubles by magnitude, the largest and
+    // Inf as Inf or NaN, NaN as NaN.
+    __device__ static __forceinline__ float size(T v) { return fabsf(__int_as_float(__double2hiint(v))); }
+    __device__ static __forceinline__ bool grown(float s) { return !(s <= __uint_as_float((1023u + kGrowthExp) << 20)); }
 };
 
 // ---------------------------------------------------------------------------
@@ -186,6 +205,8 @@ struct FF {
     // A solution whose largest |x| is below 2^-100 has subnormal low words:
     // the pairs no longer carry 47 bits.
     static constexpr unsigned kTinyMag = (127u - 100u) << 23;
+    __device__ static __forceinline__ float size(T v) { return fabsf(v.h); }
+    __device__ static __forceinline__ bool grown(float s) { return !(s <= __uint_as_float((127u + kGrowthExp) << 23)); }
 
     __device__ static __forceinline__ T in(const double* p) { return split(*p); }
     __device__ static __forceinline__ T in_ro(const double* p) { return split(__ldg(p)); }

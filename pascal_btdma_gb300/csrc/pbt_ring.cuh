@@ -155,9 +155,13 @@ __host__ __device__ constexpr bool ring_step() {
     return Num::kConv && M >= 4;
 }
 
-template <class Num, int M, bool Transposed>
+// Guard: as thomas_cols_body (pbt_cols.cuh), but y stays in D and d is kept in
+// g.aw's first planes (`saved` of k_redo_cols): 16384 x 512, FP64 m = 4, 5590 us
+// unguarded, 5660 so, 5750 with y there.
+template <class Num, int M, bool Transposed, bool Guard>
 __global__ void __launch_bounds__(256, 2) k_thomas_ring(const __grid_constant__ ThomasMaps maps, const SolveArgs g,
-                                                        const LineStrides ls, int row_first, int slots) {
+                                                        const LineStrides ls, int row_first, int slots,
+                                                        unsigned char* redo) {
     using T = typename Num::T;
     using Acc = typename Num::Acc;
     extern __shared__ __align__(128) double ring[];  // slots x warps x M x 32, then C'_{q-1} and y_{q-1}
@@ -211,6 +215,7 @@ __global__ void __launch_bounds__(256, 2) k_thomas_ring(const __grid_constant__ 
         }
     };
     unsigned bad = 0, amax = 0;
+    [[maybe_unused]] float size = 0.f;  // of C'
     for (int q = 0; q < N; ++q) {
         if constexpr (ring_step<Num, M>()) asm volatile("barrier.sync 1, %0;" ::"r"(active * 32) : "memory");
         const size_t o = (size_t)q * rs;
@@ -221,6 +226,12 @@ __global__ void __launch_bounds__(256, 2) k_thomas_ring(const __grid_constant__ 
             take(v);
 #pragma unroll
             for (int i = 0; i < M; ++i) xd[i] = Num::acc(Num::in_rhs(&v[i]));
+            if constexpr (Guard) {
+                if (live) {
+#pragma unroll
+                    for (int i = 0; i < M; ++i) __stcs(g.aw + o0 + o + (size_t)i * plane0, v[i]);
+                }
+            }
         }
 #pragma unroll
         for (int j = 0; j < M; ++j) {
@@ -279,6 +290,7 @@ __global__ void __launch_bounds__(256, 2) k_thomas_ring(const __grid_constant__ 
             } else {
 #pragma unroll
                 for (int i = 0; i < M; ++i, pw += plane) {
+                    if constexpr (Guard) size = max_nan(size, Num::size(xj[i]));
                     if (live) {
                         if (raw || !Num::kConv)
                             Num::sts(pw, xj[i]);
@@ -321,15 +333,22 @@ __global__ void __launch_bounds__(256, 2) k_thomas_ring(const __grid_constant__ 
         if (lane == 0) atomicAdd(g.status, kStallMark);
         return;
     }
+    if constexpr (Guard) {
+        if (live && (bad != 0 || Num::grown(size))) {
+            redo[sys] = 1;
+            return;
+        }
+    }
     if (live) report_status(g.status, bad | range_bits<Num>(amax, true));
 }
 
 // Consumer threads a CTA: as in_step_tpb, at most 224 (with the producer, two
 // CTAs of 256 threads of 128 registers an SM), so that the CTAs make whole
 // waves; as many ring slots as two CTAs an SM leave shared memory for.
-template <class Num, int M, bool Transposed>
-cudaError_t launch_ring(const SolveArgs& g, const LineStrides& ls, const ThomasMaps& maps, int row_first) {
-    const auto kernel = k_thomas_ring<Num, M, Transposed>;
+template <class Num, int M, bool Transposed, bool Guard>
+cudaError_t launch_ring(const SolveArgs& g, const LineStrides& ls, const ThomasMaps& maps, int row_first,
+                        unsigned char* redo) {
+    const auto kernel = k_thomas_ring<Num, M, Transposed, Guard>;
     const long long sms = g.sms > 0 ? g.sms : 1, cap = 224;
     const long long waves = (g.nsys + cap * sms - 1) / (cap * sms);
     const int warps = (int)((((long long)g.nsys + waves * sms - 1) / (waves * sms) + 31) / 32);
@@ -342,16 +361,26 @@ cudaError_t launch_ring(const SolveArgs& g, const LineStrides& ls, const ThomasM
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     const unsigned grid = (unsigned)(((g.nsys + 31) / 32 + warps - 1) / warps);
-    kernel<<<grid, 32 * (warps + 1), smem, g.stream>>>(maps, g, ls, row_first, (int)slots);
+    kernel<<<grid, 32 * (warps + 1), smem, g.stream>>>(maps, g, ls, row_first, (int)slots, redo);
     return cudaGetLastError();
 }
-template <class Num, int M>
-cudaError_t launch_thomas_ring(const SolveArgs& g, const LineStrides& ls, const ThomasMaps& maps, int row_first) {
-    return launch_ring<Num, M, false>(g, ls, maps, row_first);
+// Guarded plans take the ring in FP64 from m = 4 on only.
+template <class Num, int M, bool Transposed>
+cudaError_t launch_ring(const SolveArgs& g, const LineStrides& ls, const ThomasMaps& maps, int row_first,
+                        unsigned char* redo) {
+    if (redo == nullptr) return launch_ring<Num, M, Transposed, false>(g, ls, maps, row_first, redo);
+    if constexpr (!Num::kConv && M >= 4) return launch_ring<Num, M, Transposed, true>(g, ls, maps, row_first, redo);
+    return cudaErrorNotSupported;
 }
 template <class Num, int M>
-cudaError_t launch_transposed_ring(const SolveArgs& g, const LineStrides& ls, const ThomasMaps& maps) {
-    return launch_ring<Num, M, true>(g, ls, maps, 1);
+cudaError_t launch_thomas_ring(const SolveArgs& g, const LineStrides& ls, const ThomasMaps& maps, int row_first,
+                               unsigned char* redo) {
+    return launch_ring<Num, M, false>(g, ls, maps, row_first, redo);
+}
+template <class Num, int M>
+cudaError_t launch_transposed_ring(const SolveArgs& g, const LineStrides& ls, const ThomasMaps& maps,
+                                   unsigned char* redo) {
+    return launch_ring<Num, M, true>(g, ls, maps, 1, redo);
 }
 
 }  // namespace pbt
