@@ -616,25 +616,28 @@ bool method_free(const pbt_plan_desc& d) {
 // Whether such a plan solves its lines from both ends at once (the twisted form
 // of pbt_cols.cuh: half the chain of one segment at the same arithmetic, against
 // the two-stage method's 2.4 times): while its pairs of warps are resident
-// together (three rounds of them for m <= 3, whose rows are short), if one
-// segment pays at all or the chain of half the rows ends before the two-stage
-// method's chain and work (ColsCost).  us, segments / one segment -> twisted:
-// float-float m = 3, 6500 x 512 in 16 1121 / 1013 -> 632, 1500 261 / 850 -> 425
-// (stays in segments); m = 5, 1500 x 256 in 3 627 / 568 -> 329, 8000 x 512 in 16
-// 3507 / 2527 -> 2537 (stays in one); FP64 m = 4, 4000 x 512 in 16 2333 / 2233
-// -> 1961, 8000 4403 / 4549 -> 5872 (past residency); m = 8, 800 x 512 in 16
-// 5035 / 6325 -> 3501.
+// together (three rounds of them for m = 2, whose rows are short and which has no
+// one-segment form here), if one segment pays at all or the chain of half the rows
+// ends before the two-stage method's chain and work (ColsCost), with 15 % to spare:
+// the model's chain is that of a nearly empty SM.  Not m = 1, whose segments need
+// the fewest bytes a row (FP64 8000 x 2048 in 64 642, twisted 871).
+// us, segments / one segment / twisted, 512 rows in 16 but where told:
+// float-float m = 2, 8800 432 / 583 / 352; m = 3, 2000 286 / 616 / 332 (stays in
+// segments), 4400 710 / 651 / 405, 8800 1320 / 758 / 778, 12347 x 301 in 3 897 /
+// 629 / 663 (one); m = 4, 2000 565 / 1135 / 639 (stays); m = 5, 2000 1370 / 1211 /
+// 745, 8800 3676 / 2550 / 2992 (one); FP64 m = 3, 4400 1482 / 1260 / 951, 11000 2746
+// / 2414 / 3189 (one); m = 4, 4400 2334 / 2198 / 1957; m = 8, 700 4977 / 6377 / 3498.
 bool twisted_pays(const pbt_plan_desc& d, int sms) {
-    if (!method_free(d) || d.threads_per_block) return false;
+    if (!method_free(d) || d.threads_per_block || d.m < 2) return false;
     const int arith = arith_of(d.precision), per = 32 / (d.m + 1);
     const long long n = sms > 0 ? sms : 152, warps = 2LL * ((d.nsys + per - 1) / per);
-    if (!cols_pay(arith, d.m, d.nsys, false, sms) || warps > n * (d.m <= 3 ? 48 : d.m <= 6 ? 16 : 12)) return false;
+    if (!cols_pay(arith, d.m, d.nsys, false, sms) || warps > n * (d.m <= 2 ? 48 : d.m <= 6 ? 16 : 12)) return false;
     if (one_segment_pays(d, sms)) return true;
     const pbt::ColsCost& c = arith == kFF ? pbt::kColsFF : pbt::kColsF64;
     const double rows = 1e-3 * d.nsys * d.nrow, chain = c.chain[d.m - 1];
     const double both_ends = std::fmax(0.5 * d.nrow * chain, rows * c.row[d.m - 1]);
     const double segments = std::fmax((1.8 * d.nrow / d.nseg + 2.0 * d.nseg + 12.0) * chain, rows * c.segmented[d.m - 1]);
-    return both_ends < segments;
+    return 1.15 * both_ends < segments;
 }
 
 // The local-stage and update launches put the segments in gridDim.y.
