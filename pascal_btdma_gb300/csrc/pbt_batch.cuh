@@ -248,8 +248,7 @@ cudaError_t launch_batch(const BatchArgs& ba, int warps, cudaStream_t s, int* gr
         cudaError_t e = cudaGetDevice(&dev);
         if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         const size_t smem = (size_t)32 * warps * batch_slots<Num, M>() * sizeof(double);
-        if (e == cudaSuccess && smem > 48u * 1024u)
-            e = cudaFuncSetAttribute(k_batch_local<Num, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e == cudaSuccess) e = allow_smem(k_batch_local<Num, M>, smem);
         if (e == cudaSuccess)
             e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_local<Num, M>, 32 * warps, smem);
         if (e != cudaSuccess) return e;

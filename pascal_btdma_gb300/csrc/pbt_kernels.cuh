@@ -606,6 +606,17 @@ int kernel_regs(K* k) {
     return a.numRegs > 0 ? a.numRegs : 255;
 }
 
+// Lets a launch of kernel k take `smem` bytes of dynamic shared memory.  The limit
+// belongs to the kernel, not to the launch: it is always raised to the same value
+// (all that a CTA may have beside 1 KB of static arrays), so that no other host
+// thread's smaller launch lowers it between this call and the launch.
+template <class K>
+cudaError_t allow_smem(K* k, size_t smem) {
+    constexpr int kLimit = 226 * 1024;
+    if (smem <= 48u * 1024u) return cudaSuccess;
+    return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kLimit);
+}
+
 inline int in_step_cap(size_t smem_thread, int regs) {
     int cap = 256;
     while (cap > 32 && (2 * ((size_t)cap * smem_thread + 1024) > 228u * 1024u || 2L * cap * regs > 65536L)) cap -= 32;
@@ -2778,11 +2789,7 @@ cudaError_t launch_thomas(const SolveArgs& g) {
     const int tpb =
         kStep ? in_step_tpb(g, g.nsys, kSmemThread, regs) : (g.tpb < kThomasThreads ? g.tpb : kThomasThreads);
     const size_t smem = (size_t)tpb * kSmemThread;
-    if (smem > 48u * 1024u) {
-        const cudaError_t e =
-            cudaFuncSetAttribute(k_thomas<Num, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
+    if (const cudaError_t e = allow_smem(k_thomas<Num, M>, smem); e != cudaSuccess) return e;
     k_thomas<Num, M><<<grid_x(g.nsys, tpb), tpb, smem, g.stream>>>(g);
     return cudaGetLastError();
 }
@@ -2796,11 +2803,7 @@ cudaError_t launch_thomas_lines(const SolveArgs& g, const LineStrides& ls) {
         const int tpb = thomas_in_step<Num, M>() ? in_step_tpb(g, g.nsys, kSmemThread, regs)
                                                  : (g.tpb < kThomasThreads ? g.tpb : kThomasThreads);
         const size_t smem = (size_t)tpb * kSmemThread;
-        if (smem > 48u * 1024u) {
-            const cudaError_t e =
-                cudaFuncSetAttribute(k_thomas_lines<Num, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess) return e;
-        }
+        if (const cudaError_t e = allow_smem(k_thomas_lines<Num, M>, smem); e != cudaSuccess) return e;
         k_thomas_lines<Num, M><<<grid_x(g.nsys, tpb), tpb, smem, g.stream>>>(g, ls);
         return cudaGetLastError();
     }
@@ -2819,11 +2822,7 @@ cudaError_t launch_thomas_cyclic(const SolveArgs& g) {
             tpb = in_step_tpb(g, g.nsys, cyclic_slots<Num, M>() * sizeof(double), regs);
         }
         const size_t smem = (size_t)tpb * cyclic_slots<Num, M>() * sizeof(double);
-        if (smem > 48u * 1024u) {
-            const cudaError_t e = cudaFuncSetAttribute(k_thomas_cyclic<Num, M>,
-                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess) return e;
-        }
+        if (const cudaError_t e = allow_smem(k_thomas_cyclic<Num, M>, smem); e != cudaSuccess) return e;
         k_thomas_cyclic<Num, M><<<grid_x(g.nsys, tpb), tpb, smem, g.stream>>>(g);
         return cudaGetLastError();
     }
@@ -2838,11 +2837,7 @@ cudaError_t launch_modi(const SolveArgs& g) {
                               : (g.tpb < kThomasThreads ? g.tpb : kThomasThreads);
         const int tpb = segment_tpb(g, one, kStep ? in_step_cap(kSmemThread, regs) : one, regs, kStep ? 20 : 5);
         const size_t smem = (size_t)tpb * kSmemThread;
-        if (smem > 48u * 1024u) {
-            const cudaError_t e =
-                cudaFuncSetAttribute(k_modi_lu<Num, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess) return e;
-        }
+        if (const cudaError_t e = allow_smem(k_modi_lu<Num, M>, smem); e != cudaSuccess) return e;
         dim3 grid(grid_x(g.nsys, tpb), (unsigned)g.nseg);
         k_modi_lu<Num, M><<<grid, tpb, smem, g.stream>>>(g);
     } else {

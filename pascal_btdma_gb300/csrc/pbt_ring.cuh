@@ -358,8 +358,7 @@ cudaError_t launch_ring(const SolveArgs& g, const LineStrides& ls, const ThomasM
     size_t slots = (budget - fixed) / slot;
     if (slots > kRingSlots) slots = kRingSlots;
     const size_t smem = fixed + slots * slot;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
+    if (const cudaError_t e = allow_smem(kernel, smem); e != cudaSuccess) return e;
     const unsigned grid = (unsigned)(((g.nsys + 31) / 32 + warps - 1) / warps);
     kernel<<<grid, 32 * (warps + 1), smem, g.stream>>>(maps, g, ls, row_first, (int)slots, redo);
     return cudaGetLastError();
