@@ -124,8 +124,9 @@ typedef struct pbt_plan_desc {
     double tol;            /* PBT_PREC_FP32_REFINE: target relative correction size */
     int max_iter;          /* PBT_PREC_FP32_REFINE: refinement iteration cap */
     int threads_per_block; /* 0 = choose automatically (float-float kernels whose
-                              CTAs keep their warps on the same row take up to 256
-                              threads); else a multiple of 32 in 32..128, used as is */
+                              CTAs keep their warps on the same row and the ring's
+                              take up to 256 threads, one lane per block column up
+                              to 512); else a multiple of 32 in 32..128, used as is */
     int reserved[7];
 } pbt_plan_desc;
 
@@ -287,11 +288,13 @@ int pbt_solve_noncyclic_noalloc(double* a, double* b, double* c, double* d,
  *   dL/dA_q = -lambda_q x_{q-1}^T,  dL/dB_q = -lambda_q x_q^T,  dL/dC_q = -lambda_q x_{q+1}^T,
  * with dL/dA_0 = dL/dC_{nrow-1} = 0.  x is the forward solution and a, b, c
  * the forward blocks, unchanged (the plan must not be PBT_FLAG_INPLACE).
- * nseg = 1 (every m): one fused kernel solves M^T lambda = g by block Thomas
- * on the transposed blocks, read in place, and forms the gradient blocks in
- * its backward sweep.  nseg > 1: M^T's blocks are materialised in plan
- * workspace (allocated by the first such call), solved by the plan's forward
- * method, and the gradients formed in one more pass.  Precision fp64 or ff. */
+ * Plans solved in one segment or from both ends read the transposed blocks in
+ * place: by the forward solve's own kernels and one more pass for the gradients,
+ * or, where the forward solve has one thread per system, by one fused kernel that
+ * forms the gradient blocks in its backward sweep.  Plans that run the two-stage
+ * method on their segments materialise M^T's blocks in plan workspace (allocated
+ * by the first such call), solve them by it, and form the gradients in one more
+ * pass.  Precision fp64 or ff. */
 int pbt_adjoint_noncyclic(pbt_plan* plan, const double* a, const double* b, const double* c,
                           const double* x, double* g, double* da, double* db, double* dc,
                           int m, int nsys, int nrow, void* stream);

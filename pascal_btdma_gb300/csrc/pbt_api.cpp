@@ -588,7 +588,7 @@ bool fills_gpu(int nsys, int sms) {
 // with one lane per block column (pbt_cols.cuh), takes no longer than the
 // two-stage method's 2.4 times the arithmetic (systems an SM; GB300, us,
 // segments -> one segment):
-//   float-float m = 3, 12347 x 301 in 3 897 -> 709, 3000 x 512 in 16 513 -> 627
+//   float-float m = 3, 12347 x 301 in 3 897 -> 629, 3000 x 512 in 16 513 -> 627
 //     (line at 30); m = 5, 2500 x 512 in 16 1598 -> 1201, 1500 984 -> 1100 (14);
 //     m = 6, 1300 2161 -> 1894, 900 1594 -> 1862 (8); m = 8, 1600 3691 -> 3352,
 //     1000 2385 -> 3306 (9);
@@ -596,7 +596,7 @@ bool fills_gpu(int nsys, int sms) {
 //     in 16 1459 -> 1228 (22; 1024 x 128 in 4 150 -> 301); m = 4, 12000 5743 ->
 //     5409, 8000 4401 -> 4547 (78); m = 5, 3000 2872 -> 2840, 2000 2283 -> 2677
 //     (18); m = 8, 1300 6550 -> 6401, 800 5031 -> 6323, 4096 x 1024 in 4 39237
-//     -> 30475 (8).
+//     -> 25075 (8).
 // m <= 2 keeps its segments up to fills_gpu's line (FP64 m = 2, 14000 x 512 in
 // 16 1222 -> 1686; float-float 13000 626 -> 628).
 bool one_segment_pays(const pbt_plan_desc& d, int sms) {

@@ -94,7 +94,8 @@ template <class Num, int M> cudaError_t launch_update(const SolveArgs& g);
 // method, by m = 1 .. 10, from sweeps on a GB300: us a row of a line's chain, ns
 // a row of a batch that fills the GPU, ns a row of the local stage and update of
 // a batch that does not quite.  They decide between methods, so what counts is
-// their order, not the last tenth.
+// their order, not the last tenth.  (segmented, float-float: from m = 6 on the local
+// stage spills at its register cap, 668 bytes a thread at m = 6, 92 at m = 5.)
 struct ColsCost {
     double chain[10], row[10], segmented[10];
 };
