@@ -163,7 +163,7 @@ void pbt_plan_desc_init(pbt_plan_desc* desc);
  * at once, where that is faster.  Those orders of elimination invert other blocks
  * than the nseg segments do, so a line that they do not suit -- they meet a zero
  * pivot, or an element of C'_q = R_q^{-1} C_q (from the last row on, of R_q^{-1}
- * A_q) above 2^10; a singular or tiny last block is an example -- is solved again
+ * A_q) above 2^6; a singular or tiny last block is an example -- is solved again
  * in its segments, with their x and their report.  Block diagonally dominant lines
  * never are; a batch most of whose lines are is solved faster with
  * PBT_FLAG_REFERENCE_METHOD.  The workspace is that of the segments.

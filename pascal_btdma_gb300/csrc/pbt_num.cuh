@@ -60,9 +60,11 @@ __device__ __forceinline__ double dsel(unsigned s, double x, double y) {
 // Solves whose order of elimination the library chose (Guard, pbt_cols.cuh) keep
 // a line's solution only if no element of its C' blocks passed 2^kGrowthExp: what
 // an element loses to a larger one in the sums of the next row, and in the
-// substitution back, is at most that factor.  C' of a block diagonally dominant
-// line stays below 1.
-constexpr unsigned kGrowthExp = 10;
+// substitution back, is at most that factor: 2^6 times float-float's 1e-14 is
+// inside the 1e-12 that both arithmetics keep to (last blocks that grow to 180,
+// redone from 2^10 on: 2.5e-12 to 6.4e-12).  C' of a block diagonally dominant line
+// stays below 1.
+constexpr unsigned kGrowthExp = 6;
 // The larger value; NaN if either is.
 __device__ __forceinline__ float max_nan(float a, float b) {
     float r;

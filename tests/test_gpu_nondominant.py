@@ -118,6 +118,31 @@ def test_every_line_of_a_batch_that_is_not_dominant(cuda, prec):
     check_lines(dense(a, b, c, s), vectors(x, s), vectors(d, s), prec)
 
 
+@pytest.mark.parametrize("prec", ["fp64", "ff"])
+@pytest.mark.parametrize("m,nsys,nseg", [(2, 300, 2), (3, 700, 4), (5, 500, 2), (8, 300, 2)])
+@pytest.mark.parametrize("scale", [3e-2, 3e-3, 3e-4, 3e-6])
+def test_small_last_blocks_keep_the_parity_bound(cuda, prec, m, nsys, nseg, scale):
+    """Element growth of any size, up to the one from which a line is redone and past
+    it: the bound of both arithmetics (1e-12) holds, as in the segments."""
+    nrow = 9 * nseg
+    a, b, c, d = (x.view(m, -1, nrow, nsys) for x in batch(m, nsys, nrow, seed=m))
+    d = d.view(m, nrow, nsys)
+    s = torch.arange(nsys, device=cuda)
+    spoil(a, b, c, "last", s)
+    b[:, :, -1] = scale * (a[:, :, -1] + m * torch.eye(m, dtype=a.dtype, device=cuda)[:, :, None])
+    x = d.clone()
+    with pbt.BtdmaGpuPlan() as plan:
+        plan.create(m, nsys, nrow, nseg, precision=prec)
+        pbt.solve_noncyclic(plan, a, b, c, x, m, nsys, nrow)
+        assert plan.status() == 0
+    M = dense(a, b, c, s)
+    kappa = M.abs().sum(-1).amax(-1) * torch.linalg.inv(M).abs().sum(-1).amax(-1)
+    assert float(kappa.max()) < 100  # what is lost is lost to growth
+    ref = torch.linalg.solve(M, vectors(d, s).unsqueeze(-1)).squeeze(-1)
+    err = (vectors(x, s) - ref).abs().amax(-1) / ref.abs().amax(-1)
+    assert float(err.max()) <= 1e-12
+
+
 def columns_batch(seed):
     """Systems of m = 1..6 and N = 16..60, so many of each that the plan solves all
     in one launch by block columns; their last tiles have 1, 31 or 32 lanes."""
